@@ -191,6 +191,14 @@ __global__ void __launch_bounds__(1024) avoid_update_kernel(AvoidParams a) {
     }
 }
 
+// Dynamic shared memory of a CTA: the tier's layout, then `weights` draw weights (0: a kernel without a draw); the
+// FP64 tiers up to 32 columns lay the pair sweep's tables over the weights.
+static size_t cta_smem_bytes(int kpm, int prec, int weights) {
+    const size_t tables = (prec == PE_PRECISION_F64 && kpm <= NARROW) ? sizeof(PairTables<NARROW>) : 0;
+    const size_t w = (size_t)weights * sizeof(double);
+    return smem_fixed_bytes_for(kpm, prec) + (w > tables ? w : tables);
+}
+
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 static size_t split_bytes(int64_t S, int nch) {
     return nch > 0 ? (size_t)S * nch * MAXN * sizeof(double2) + (size_t)S * sizeof(int) : 0;
@@ -205,7 +213,7 @@ extern "C" int pe_max_modes(int block_threads) {
     (void)block_threads;
     const int cap = max_smem_optin();
     if (cap <= 0) return 0;
-    return (int)((cap - (int)smem_fixed_bytes_for(NARROW)) / (int)sizeof(double));
+    return (int)((cap - (int)smem_fixed_bytes_for(NARROW, PREC_MIXED)) / (int)sizeof(double));
 }
 
 extern "C" size_t pe_chain_workspace_bytes(int64_t S) {
@@ -246,6 +254,9 @@ static int launch_prepare(void* fn, int block, size_t smem, int* grid_per_sm) {
     int occ = 0;
     PE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, smem));
     if (occ < 1) return PE_ERR_SIZE;
+    // the rest of the SM's 228 KB stays L1 (register spills, the instance's columns); a CTA holds 1 KB beside its own
+    const int carve = (int)((100 * (size_t)occ * (smem + 1024) + 228 * 1024 - 1) / (228 * 1024));
+    PE_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, carve < 100 ? carve : 100));
     *grid_per_sm = occ;
     return PE_OK;
 }
@@ -301,9 +312,8 @@ static int chain_launch(int precision, const double* d_acol, const int64_t* d_in
                                 : (block_threads ? block_threads : (bmax < 128 ? bmax : 128));
     if (block < 32 || block > 256 || block > bmax || (block & 31)) return PE_ERR_ARG;
     if (!warp_mode && block < ncols) return PE_ERR_ARG;
-    const size_t smem_fix = smem_fixed_bytes_for(kpm, precision);
     const size_t smem = warp_mode ? warp_smem_bytes(precision, tpl, kpm, block / 32)
-                                  : smem_fix + (size_t)m_max * sizeof(double);
+                                  : cta_smem_bytes(kpm, precision, m_max);
     const int cap = max_smem_optin();
     if (cap <= 0) return PE_ERR_CUDA;
     if (smem > (size_t)cap) return PE_ERR_SIZE;
@@ -355,8 +365,8 @@ static int chain_launch(int precision, const double* d_acol, const int64_t* d_in
         if (!fpart[q] || !fdraw[q]) return PE_ERR_SIZE;
         int per_part = 0, per_draw = 0;
         const int pq = q == 0 ? precision : PE_PRECISION_F64;
-        const size_t sdraw = smem_fixed_bytes_for(kpm, pq) + (size_t)m_max * sizeof(double);
-        if ((rc = launch_prepare(fpart[q], block, smem_fixed_bytes_for(kpm, pq), &per_part)) != PE_OK) return rc;
+        const size_t sdraw = cta_smem_bytes(kpm, pq, m_max);
+        if ((rc = launch_prepare(fpart[q], block, cta_smem_bytes(kpm, pq, 0), &per_part)) != PE_OK) return rc;
         if ((rc = launch_prepare(fdraw[q], block, sdraw, &per_draw)) != PE_OK) return rc;
         gpart[q] = items < (int64_t)sms * per_part ? items : (int64_t)sms * per_part;
         gdraw[q] = nq < (int64_t)sms * per_draw ? nq : (int64_t)sms * per_draw;
@@ -375,9 +385,9 @@ static int chain_launch(int precision, const double* d_acol, const int64_t* d_in
             sp.pass = q;
             const int pq = q == 0 ? precision : PE_PRECISION_F64;
             PE_CUDA_TRY(cudaLaunchKernel(fpart[q], dim3((unsigned)gpart[q]), dim3(block), sargs,
-                                         smem_fixed_bytes_for(kpm, pq), st));
+                                         cta_smem_bytes(kpm, pq, 0), st));
             PE_CUDA_TRY(cudaLaunchKernel(fdraw[q], dim3((unsigned)gdraw[q]), dim3(block), sargs,
-                                         smem_fixed_bytes_for(kpm, pq) + (size_t)m_max * sizeof(double), st));
+                                         cta_smem_bytes(kpm, pq, m_max), st));
         }
     }
     return PE_OK;
@@ -542,7 +552,7 @@ extern "C" int pe_cofactors_rows(int precision, const double* d_a, const int64_t
     cudaStream_t st = (cudaStream_t)stream;
     PE_CUDA_TRY(cudaMemsetAsync(d_workspace, 0, WS_BYTES, st));
     if (S == 0) return PE_OK;
-    const size_t smem = smem_fixed_bytes_for(kpm, precision);
+    const size_t smem = cta_smem_bytes(kpm, precision, 0);
     int per_sm = 0;
     int rc = launch_prepare(fn, block, smem, &per_sm);
     if (rc != PE_OK) return rc;
@@ -577,7 +587,7 @@ extern "C" int pe_split_slots(int precision, int n_stride, int block_threads, in
     const int block = block_threads ? block_threads : (bmax < 128 ? bmax : 128);
     if (block < 32 || block > 256 || block > bmax || (block & 31)) return PE_ERR_ARG;
     int per_sm = 0, dev = 0, sms = 0;
-    const int rc = launch_prepare(fn, block, smem_fixed_bytes_for(kpm, precision), &per_sm);
+    const int rc = launch_prepare(fn, block, cta_smem_bytes(kpm, precision, 0), &per_sm);
     if (rc != PE_OK) return rc;
     PE_CUDA_TRY(cudaGetDevice(&dev));
     PE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

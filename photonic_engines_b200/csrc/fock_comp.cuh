@@ -242,7 +242,7 @@ __device__ void sweep_comp(SM& sm) {
     double ar[2 * KA], ai[2 * KA];
 #pragma unroll
     for (int j = 0; j < 2 * KA; ++j) { ar[j] = 0.0; ai[j] = 0.0; }
-    for (int64_t hw = sm.lane0 + wl0; hw < H; hw += (int64_t)lanes * sm.lane_mult) {
+    for (int64_t hw = sm.chunk * lanes + wl0; hw < H; hw += (int64_t)lanes * sm.lane_mult) {
         double wlane;
         int64_t hl = hw + (lane - wl0);
         const bool live = hl < H;

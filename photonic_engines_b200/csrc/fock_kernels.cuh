@@ -202,8 +202,10 @@ __device__ __forceinline__ void exclusive_product(T (&v)[GL]) {
 // the middle block; what does not fit the schedules joins the lanes.  The ranking takes one ballot per
 // distinct radix value, and every digit's table entries are written by the lane of its rank, so only
 // the choice of the three splits walks the ranks one by one (in registers, read by shuffles).
+// pair_lanes > 0: take two digits of multiplicity 1 out for the pair sweep of that many lanes, when there are
+// two; N then counts its blocks of four terms.
 template <class SM>
-__device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid_max) {
+__device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid_max, int pair_lanes = 0) {
     auto& pl = sm.plan;
     constexpr int GL = (SM::NKMAX + 31) / 32;          // groups (and ranks) per lane: index lane + 32 q, q < GL
     const unsigned full = 0xffffffffu;
@@ -217,6 +219,19 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
         const unsigned oddmask = __ballot_sync(full, g < D && (sm.gmul[g < D ? g : 0] & 1));
         if (oddmask) halved = 32 * q + 31 - __clz(oddmask);
     }
+    // the pair sweep's digits u, v: the first two groups of multiplicity 1 (the halved one aside)
+    int gu = -1, gv = -1;
+    if (pair_lanes > 0) {
+#pragma unroll
+        for (int q = 0; q < GL; ++q) {
+            const int g = lane + 32 * q;
+            unsigned ones = __ballot_sync(full, g < D && g != halved && sm.gmul[g < D ? g : 0] == 1);
+            if (ones && gu < 0) { gu = 32 * q + __ffs(ones) - 1; ones &= ones - 1u; }
+            if (ones && gv < 0) gv = 32 * q + __ffs(ones) - 1;
+        }
+        if (gv >= 0) lanes = pair_lanes;
+        else gu = -1;                                  // fewer than two: the sweep term by term
+    }
     int R[GL];
     bool active[GL];
 #pragma unroll
@@ -224,7 +239,7 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
         const int g = lane + 32 * q;
         const int M = g < D ? sm.gmul[g] : 0;
         R[q] = g < D ? (g == halved ? (M + 1) / 2 : M + 1) : 1;
-        active[q] = R[q] >= 2;
+        active[q] = R[q] >= 2 && g != gu && g != gv;
     }
     // ranks by (radix, group): the groups of the smallest remaining radix take the next ranks in group order
     unsigned rem[GL];
@@ -319,7 +334,7 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
             if (p >= nhi + nin && p < nhi + nin + nmid) pl.Pmid[kd - nin] = pmid[q];
         }
         const int g = lane + 32 * q;                   // fixed digits: after the active ones, in group order
-        const bool fixed = g < D && !active[q];
+        const bool fixed = g < D && !active[q] && g != gu && g != gv;
         const unsigned fm = __ballot_sync(full, fixed);
         if (fixed) {
             const int kd = na + nfix + __popc(fm & below);
@@ -329,7 +344,16 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
         }
         nfix += __popc(fm);
     }
+    if (gv >= 0 && lane < 2) {                         // u, v: the last two digits
+        const int kd = na + nfix + lane;
+        pl.R[kd] = 2;
+        pl.M[kd] = 1;
+        pl.drow[kd] = sm.grow[lane == 0 ? gu : gv];
+    }
     if (lane == 0) {
+        pl.pairs = gv >= 0;
+        pl.pu = na + nfix;
+        pl.pv = na + nfix + 1;
         pl.N = N; pl.H = N / ((long long)Lin * Lmid); pl.Lin = Lin; pl.Lmid = Lmid;
         pl.K = K; pl.K1 = K1; pl.D = D;
         pl.nin = nin; pl.nmid = nmid; pl.nhi = na - nin - nmid;
@@ -381,10 +405,11 @@ static __device__ __forceinline__ unsigned char gray_entry(const PL& pl, int d0,
 // All threads.  Element (rho, j) of the instance is A[rho * rs + j * cs].  kh > 0 (mixed form with
 // paired FP32 sweeps, kh columns per thread): row kd of B32 is written as float4 slots
 // q = h * kh/2 + c holding (re b_j1, re b_j2, im b_j1, im b_j2) of 2b, j1 = h * kh + c, j2 = j1 + kh/2 —
-// the two columns whose product chains one paired instruction advances together.
+// the two columns whose product chains one paired instruction advances together.  pair_kh > 0 (a step that runs
+// the pair sweep): column h * pair_kh + r of B goes to position r * 2^tl + h of its row.
 template <class SM>
 static __device__ void prepare_step(SM& sm, const double2* __restrict__ A, int64_t rs, int64_t cs, bool mixed,
-                                    int kh = 0) {
+                                    int kh = 0, int pair_kh = 0, int tl = 0) {
     constexpr int NK = SM::NKMAX;
     constexpr bool narrow = SM::NK32 == NK;           // the wide layout has no FP32 copy (FP64 only)
     const auto& pl = sm.plan;
@@ -393,13 +418,15 @@ static __device__ void prepare_step(SM& sm, const double2* __restrict__ A, int64
     // per GB elements instead of one per element)
     constexpr int GB = 8;
     const int nel = pl.D * NK;
+    if (pair_kh == 0) { pair_kh = NK; tl = 0; }
     for (int base = tid; base < nel; base += T * GB) {
         double2 v[GB];
 #pragma unroll
         for (int g = 0; g < GB; ++g) {
             const int idx = base + g * T;
-            const bool ok = idx < nel && idx % NK < pl.K;
-            const int kd = ok ? idx / NK : 0, j = ok ? idx % NK : 0;      // in range even when not loaded
+            const int pos = idx % NK, r = pos >> tl, col = (pos - (r << tl)) * pair_kh + r;
+            const bool ok = idx < nel && r < pair_kh && col < pl.K;
+            const int kd = ok ? idx / NK : 0, j = ok ? col : 0;           // in range even when not loaded
             v[g] = ok ? A[(int64_t)pl.drow[kd] * rs + (int64_t)sm.cols[j] * cs] : make_double2(0.0, 0.0);
         }
 #pragma unroll
@@ -847,8 +874,9 @@ static __device__ __forceinline__ uint64_t lane_digits(const PL& pl, int64_t hl,
 
 // Column sums of one lane at a given digit state, FP64: s_j = sum_kd (M_kd - 2 v_kd) B[kd][j] with the
 // inner digits at their start (0) or end (vend) state, the middle digits at middle index pm and the
-// high digits of the lane (packed by lane_digits; more than 12 high digits are decoded from hl).
-template <int KH, class SM>
+// high digits of the lane (packed by lane_digits; more than 12 high digits are decoded from hl).  The thread's
+// columns are at c0, c0 + STEP, ... of the rows of B.
+template <int KH, int STEP = 1, class SM>
 __device__ __forceinline__ void lane_sums(const SM& sm, int c0, bool inner_end, int pm, int64_t hl, uint64_t hpack,
                                           double (&xr)[KH], double (&xi)[KH]) {
     const auto& pl = sm.plan;
@@ -860,7 +888,7 @@ __device__ __forceinline__ void lane_sums(const SM& sm, int c0, bool inner_end, 
         const double c = (double)(pl.M[kd] - 2 * v);
         const double2* b = &sm.B[kd][c0];
 #pragma unroll
-        for (int j = 0; j < KH; ++j) { xr[j] = fma(c, b[j].x, xr[j]); xi[j] = fma(c, b[j].y, xi[j]); }
+        for (int j = 0; j < KH; ++j) { xr[j] = fma(c, b[j * STEP].x, xr[j]); xi[j] = fma(c, b[j * STEP].y, xi[j]); }
     };
     for (int kd = 0; kd < nin; ++kd) add(kd, inner_end ? sm.plan.vend[kd] : 0);
     int par = 0;                                       // middle digits top-down (reflected Gray)
@@ -901,7 +929,7 @@ __device__ void sweep_f64(SM& sm) {
     double ar[KH], ai[KH];
 #pragma unroll
     for (int j = 0; j < KH; ++j) { ar[j] = 0.0; ai[j] = 0.0; }
-    for (int64_t hw = sm.lane0 + wl0; hw < H; hw += (int64_t)lanes * sm.lane_mult) {
+    for (int64_t hw = sm.chunk * lanes + wl0; hw < H; hw += (int64_t)lanes * sm.lane_mult) {
         double sr[KH], si[KH], wh;
         int64_t hl = hw + (lane - wl0);
         const bool live = hl < H;                          // a lane past the end repeats lane H - 1 at weight 0
@@ -942,7 +970,7 @@ __device__ void sweep_mixed(SM& sm) {
     double ar[KH], ai[KH];
 #pragma unroll
     for (int j = 0; j < KH; ++j) { ar[j] = 0.0; ai[j] = 0.0; }
-    for (int64_t hw = sm.lane0 + wl0; hw < H; hw += (int64_t)lanes * sm.lane_mult) {
+    for (int64_t hw = sm.chunk * lanes + wl0; hw < H; hw += (int64_t)lanes * sm.lane_mult) {
         double wh;
         int64_t hl = hw + (lane - wl0);
         const bool live = hl < H;
@@ -1003,24 +1031,34 @@ __device__ void sweep_mixed(SM& sm) {
         if (K <= KPv) { CALL; return; }                      \
     }
 
+// Steps of at least PAIRS_MIN columns run the pair sweep (fock_pairs.cuh) when their plan has its two digits, in
+// the kernels whose threads have 255 registers: lanes of two threads up to 20 columns, of four beyond, whatever
+// the term-by-term sweep's TPL.
+constexpr int PAIRS_MIN = 9;
+template <int TPL, int KPM>
+__host__ __device__ constexpr bool has_pairs() {
+    return PE_MAXT * PE_MINB <= 384 && TPL <= 2 && KPM >= PAIRS_MIN && KPM <= NARROW;
+}
+#ifndef PE_PAIR4
+#define PE_PAIR4 20
+#endif
+__host__ __device__ constexpr int pair_tpl(int K) { return K <= PE_PAIR4 ? 2 : 4; }
+
+// Tiers the term-by-term FP64 sweep is compiled for: all of them, but where the pair sweep runs a tier only
+// crowded steps (fewer than two modes chosen once) are left, and the kernel's last tier serves those.
+template <int TPL, int KPM, int KP>
+__host__ __device__ constexpr bool f64_tier() {
+    return KP <= KPM && (KP < PAIRS_MIN || KP == KPM || !has_pairs<TPL, KPM>());
+}
+#define PE_TIER64(KPv)                                       \
+    if constexpr (f64_tier<TPL, KPM, KPv>()) {               \
+        if (K <= KPv) { sweep_f64<KPv, TPL>(sm); return; }   \
+    }
+
 template <int TPL, int KPM, class SM>
 __device__ void dispatch_f64(SM& sm, int K) {
-    PE_TIER(4, (sweep_f64<4, TPL>(sm)))
-    PE_TIER(8, (sweep_f64<8, TPL>(sm)))
-    PE_TIER(12, (sweep_f64<12, TPL>(sm)))
-    PE_TIER(16, (sweep_f64<16, TPL>(sm)))
-    PE_TIER(20, (sweep_f64<20, TPL>(sm)))
-    PE_TIER(24, (sweep_f64<24, TPL>(sm)))
-    PE_TIER(28, (sweep_f64<28, TPL>(sm)))
-    PE_TIER(32, (sweep_f64<32, TPL>(sm)))
-    PE_TIER(36, (sweep_f64<36, TPL>(sm)))
-    PE_TIER(40, (sweep_f64<40, TPL>(sm)))
-    PE_TIER(44, (sweep_f64<44, TPL>(sm)))
-    PE_TIER(48, (sweep_f64<48, TPL>(sm)))
-    PE_TIER(52, (sweep_f64<52, TPL>(sm)))
-    PE_TIER(56, (sweep_f64<56, TPL>(sm)))
-    PE_TIER(60, (sweep_f64<60, TPL>(sm)))
-    PE_TIER(64, (sweep_f64<64, TPL>(sm)))
+    PE_TIER64(4) PE_TIER64(8) PE_TIER64(12) PE_TIER64(16) PE_TIER64(20) PE_TIER64(24) PE_TIER64(28) PE_TIER64(32)
+    PE_TIER64(36) PE_TIER64(40) PE_TIER64(44) PE_TIER64(48) PE_TIER64(52) PE_TIER64(56) PE_TIER64(60) PE_TIER64(64)
 }
 
 template <int TPL, int KPM, class SM>
@@ -1037,19 +1075,35 @@ __device__ void dispatch_mixed(SM& sm, int K) {
 }  // namespace pe
 
 #include "fock_comp.cuh"
+#include "fock_pairs.cuh"
 
 namespace pe {
+
+#define PE_PTIER(KPv)                                                                            \
+    if constexpr (KPM >= KPv) {                                                                  \
+        if (K <= KPv) { sweep_pairs_f64<KPv / pair_tpl(KPv), pair_tpl(KPv)>(sm); return; }       \
+    }
+template <int KPM, class SM>
+__device__ void dispatch_pairs(SM& sm, int K) {
+    PE_PTIER(12) PE_PTIER(16) PE_PTIER(20) PE_PTIER(24) PE_PTIER(28) PE_PTIER(32)
+}
 
 // One cofactor step of the stream held in shared memory (K1 >= 1): plan, prepare, sweep.  PREC: 0 FP64,
 // 1 mixed, 2 compensated mixed.
 template <int TPL, int KPM, int PREC, class SM>
 __device__ __forceinline__ void cofactor_step(SM& sm, const double2* A, int64_t rs, int64_t cs, int K1, int K) {
     constexpr bool MIXED = PREC == PREC_MIXED;
-    if (threadIdx.x < 32) plan_step(sm, K1, K, blockDim.x / TPL * sm.lane_mult, MIXED ? MIXED_LIN : LIN_MAX, MID_MAX);
+    constexpr bool PAIRS = PREC == PREC_F64 && has_pairs<TPL, KPM>();
+    if (threadIdx.x < 32)
+        plan_step(sm, K1, K, blockDim.x / TPL * sm.lane_mult, MIXED ? MIXED_LIN : LIN_MAX, MID_MAX,
+                  PAIRS && K >= PAIRS_MIN ? blockDim.x / pair_tpl(K) * sm.lane_mult : 0);
     __syncthreads();
     // paired FP32 sweeps (mixed form, 1- and 2-thread lanes): columns per thread of the dispatched tier
     const int kh = (MIXED && PE_PAIR32 && TPL <= 2) ? ((K + 3) / 4 * 4) / TPL : 0;
-    prepare_step(sm, A, rs, cs, MIXED, kh);
+    bool pairs = false;
+    if constexpr (PAIRS) pairs = sm.plan.pairs;
+    const int ptl = pair_tpl(K) == 2 ? 1 : 2, pkh = ((K + 3) / 4 * 4) >> ptl;
+    prepare_step(sm, A, rs, cs, MIXED, kh, pairs ? pkh : 0, ptl);
     __syncthreads();
     if constexpr (PREC == PREC_COMP) {
         prepare_comp(sm, ((K + 3) / 4 * 4) / TPL, TPL);
@@ -1058,6 +1112,14 @@ __device__ __forceinline__ void cofactor_step(SM& sm, const double2* A, int64_t 
     } else if constexpr (MIXED) {
         dispatch_mixed<TPL, KPM>(sm, K);
     } else {
+        if constexpr (PAIRS) {
+            if (pairs) {
+                prepare_pairs(sm, pkh, ptl);
+                __syncthreads();
+                dispatch_pairs<KPM>(sm, K);
+                return;
+            }
+        }
         dispatch_f64<TPL, KPM>(sm, K);
     }
 }
@@ -1184,7 +1246,7 @@ __device__ void chain_one(const ChainParams& p, SmemFor<KPM, PREC>& sm, double* 
         else sm.rows[tid] = (int)r;
     }
     if (!ok && tid == 0) sm.bad = 1;
-    if (tid == 0) { sm.ngrp = 0; sm.lane0 = 0; sm.lane_mult = 1; }
+    if (tid == 0) { sm.ngrp = 0; sm.chunk = 0; sm.lane_mult = 1; }
     __syncthreads();
     if (sm.bad) {
         if (tid == 0) record_error(p.status, p.detail, s);
@@ -1247,12 +1309,12 @@ __global__ void __launch_bounds__(PE_MAXT, PE_MINB) fock_chain_kernel(ChainParam
         if (tid == 0) {
             const unsigned long long q = atomicAdd(p.queue, 1ull);
             sm.cur = queue_stream(p, q);
-            sm.lane0 = (int64_t)q;                  // the ticket, until chain_one resets the field
+            sm.chunk = (int64_t)q;                  // the ticket, until chain_one resets the field
             sm.bad = 0;
         }
         __syncthreads();
         const int64_t s = sm.cur;
-        const bool stop_early = p.split_cap < 0 || sm.lane0 < p.split_cap;
+        const bool stop_early = p.split_cap < 0 || sm.chunk < p.split_cap;
         __syncthreads();
         if (s < 0) return;
         if (s >= p.S) {
@@ -1342,7 +1404,7 @@ __global__ void __launch_bounds__(PE_MAXT, PE_MINB) split_partial_kernel(SplitPa
         int64_t off;
         const bool live = (sp.pass == 0 || sp.flag[q] != 0) && load_state(p, sm, s, k, m, off);
         if (live) {
-            if (tid == 0) { sm.lane0 = (int64_t)i * (blockDim.x / TPL); sm.lane_mult = sp.nch; }
+            if (tid == 0) { sm.chunk = i; sm.lane_mult = sp.nch; }
             __syncthreads();
             cofactor_step<TPL, KPM, PREC>(sm, p.acol + off, 1, m, k - 1, k);
             if (tid < k) sp.partial[(q * sp.nch + i) * MAXN + tid] = sm.P[tid];
@@ -1419,7 +1481,7 @@ __global__ void __launch_bounds__(256) cofactor_kernel(const double2* __restrict
     SM& sm = *reinterpret_cast<SM*>(smem_raw);
     const int tid = threadIdx.x;
     for (int64_t s = blockIdx.x; s < S; s += gridDim.x) {
-        if (tid == 0) { sm.bad = 0; sm.ngrp = 0; sm.lane0 = 0; sm.lane_mult = 1; }
+        if (tid == 0) { sm.bad = 0; sm.ngrp = 0; sm.chunk = 0; sm.lane_mult = 1; }
         __syncthreads();
         if (tid < K) sm.cols[tid] = tid;
         if (tid < K - 1) {

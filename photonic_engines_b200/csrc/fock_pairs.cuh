@@ -1,0 +1,326 @@
+// FP64 sweep of the collapsed sum in blocks of four terms, the columns taken in pairs.
+//
+// Two digits u, v of radix 2 and multiplicity 1 (two output modes chosen once each) are taken out of the Gray
+// walk; every walked term then stands for the four sign choices of u and v around the column sums s at
+// u = v = 0.  With du = -2 B[u], dv = -2 B[v] a column's sum at digit values (x, y) is s + x du + y dv, so
+// for a pair of columns a, b
+//
+//   product   q(0,0) = s_a s_b,  q(1,0) = q(0,0) + L_u,  q(1,1) = q(1,0) + L_v + C,  q(0,1) = q(1,1) - L_u - C
+//             L_u = s_a du_b + s_b du_a + du_a du_b  (L_v alike),  C = du_a dv_b + du_b dv_a
+//   cofactor  sum_xy w_xy Y_xy (s_b + x du_b + y dv_b) = S s_b + du_b X_u + dv_b X_v
+//             Y = the product of every other pair, S = sum w Y, X_u / X_v = the terms with x = 1 / y = 1
+//
+// L_u and L_v are affine in the column sums, so they are walked by Gray updates like the sums themselves (the
+// table G holds their steps); S multiplies the column sums once per block, X_u and X_v only once per sweep.
+// Per pair and term that is 5 FP64 instructions for the products, 12 for the all-but-one products over the
+// pairs (prefix, suffix, accumulation) and 4 for the rest: 21, against 28 for two columns taken one by one.
+// Bound by the FP64 pipe (70-75 % busy inside the sweep).  Lanes of two threads with ten columns each at 20 columns
+// (eleven doubles of state per column pair and thread: 255 registers with a few spills to L1), of four threads with
+// six to eight beyond.  Measured against the term-by-term sweep: n = 20, m = 400, 2 000 streams 18.3 -> 14.2 ms;
+// n = 24, m = 576, 600 streams 128 -> 97 ms; cofactors at 28 columns (148 blocks) 329 -> 274 ms, at 32 columns
+// (16 blocks) 6.2 -> 4.9 s.
+// A thread with an odd number of columns keeps the last one as an item of its own (sum walked through the four
+// terms, 14 instructions).
+//
+// Reference: the sum itself is photonic_engines/clifford/cuda_cofactors.py:35-151 (term by term).
+#pragma once
+
+namespace pe {
+
+// A step that runs the pair sweep keeps column h KH + r of B (thread h of a lane, its r-th column) at position
+// r TPL + h of the row, so that the lane's threads read neighbouring 16-byte words: with the columns in order the
+// threads of a lane are KH 16 bytes apart, which for KH = 8 is the same banks (K = 29-32: 1.4x slower than the
+// term-by-term sweep instead of faster).
+
+// Step tables of the pair walk, in the same positions.  They take the place of the draw's weights, which are not
+// alive during a sweep.
+template <int NK>
+struct PairTables {
+    double2 G[NK][NK];         // per digit and pair (a, b): change of L_u (at a) and L_v (at b) when the sums move by B[kd]
+    double2 C[NK];             // C of the pair, at a
+};
+template <class SM>
+__device__ __forceinline__ PairTables<SM::NKMAX>& pair_tables(const SM& sm) {
+    constexpr size_t at = (sizeof(SM) + 15) & ~(size_t)15;             // smem_fixed_bytes of the layout
+    return *reinterpret_cast<PairTables<SM::NKMAX>*>(reinterpret_cast<unsigned char*>(const_cast<SM*>(&sm)) + at);
+}
+
+// All threads, after B is complete: kh columns per thread of a lane of 1 << tl threads.  Columns past K are zero in B.
+template <class SM>
+static __device__ void prepare_pairs(SM& sm, int kh, int tl) {
+    const auto& pl = sm.plan;
+    auto& pt = pair_tables(sm);
+    const int tid = threadIdx.x, T = blockDim.x, tpl = 1 << tl, kp = kh << tl;
+    const int nd = max(1, pl.nin + pl.nmid);               // row 0 is read (times zero) at a lane's first term
+    for (int idx = tid; idx < nd * kp; idx += T) {
+        const int kd = idx / kp, pos = idx % kp, r = pos >> tl;
+        if (r == kh - 1 && (kh & 1)) continue;             // the thread's single column
+        const int a = (r & 1) ? pos - tpl : pos, b = a + tpl, d = (r & 1) ? pl.pv : pl.pu;
+        const double2 ba = sm.B[kd][a], bb = sm.B[kd][b], da = sm.B[d][a], db = sm.B[d][b];
+        const double re = fma(ba.x, db.x, -(ba.y * db.y)) + fma(bb.x, da.x, -(bb.y * da.y));
+        const double im = fma(ba.x, db.y, ba.y * db.x) + fma(bb.x, da.y, bb.y * da.x);
+        pt.G[kd][pos] = make_double2(-2.0 * re, -2.0 * im);
+    }
+    for (int a = tid; a < kp; a += T) {
+        const int r = a >> tl;
+        if ((r & 1) || r == kh - 1) continue;              // the first columns of the pairs only
+        const int b = a + tpl;
+        const double2 ua = sm.B[pl.pu][a], ub = sm.B[pl.pu][b], va = sm.B[pl.pv][a], vb = sm.B[pl.pv][b];
+        const double re = fma(ua.x, vb.x, -(ua.y * vb.y)) + fma(ub.x, va.x, -(ub.y * va.y));
+        const double im = fma(ua.x, vb.y, ua.y * vb.x) + fma(ub.x, va.y, ub.y * va.x);
+        pt.C[a] = make_double2(4.0 * re, 4.0 * im);
+    }
+}
+
+// The product of the other threads' totals of a lane (TPL 2: the partner's; TPL 4: two butterfly exchanges).
+template <int TPL>
+__device__ __forceinline__ void lane_others(double xr, double xi, double& yr, double& yi) {
+    if constexpr (TPL == 1) {
+        yr = 1.0; yi = 0.0;
+    } else {
+        yr = __shfl_xor_sync(0xffffffffu, xr, 1);
+        yi = __shfl_xor_sync(0xffffffffu, xi, 1);
+        if constexpr (TPL == 4) {
+            const double gr = fma(xr, yr, -(xi * yi)), gi = fma(xr, yi, xi * yr);
+            const double br = __shfl_xor_sync(0xffffffffu, gr, 2), bi = __shfl_xor_sync(0xffffffffu, gi, 2);
+            const double nr = fma(yr, br, -(yi * bi));
+            yi = fma(yr, bi, yi * br);
+            yr = nr;
+        }
+    }
+}
+
+// P (+)= x y, complex (FIRST: P = x y).
+template <bool FIRST>
+__device__ __forceinline__ void cacc(double xr, double xi, double yr, double yi, double& Pr, double& Pi) {
+    if (FIRST) {
+        Pr = fma(xr, yr, -(xi * yi));
+        Pi = fma(xr, yi, xi * yr);
+    } else {
+        Pr = fma(xr, yr, Pr);
+        Pr = fma(-xi, yi, Pr);
+        Pi = fma(xr, yi, Pi);
+        Pi = fma(xi, yr, Pi);
+    }
+}
+__device__ __forceinline__ void cmul_by(double& xr, double& xi, double yr, double yi) {
+    const double nr = fma(xr, yr, -(xi * yi));
+    xi = fma(xr, yi, xi * yr);
+    xr = nr;
+}
+
+// The items [LO, HI) of one half, y = the product of everything else: P[p] += y prod of the half's other items.
+template <int LO, int HI, int NP, int NI, bool FIRST>
+__device__ __forceinline__ void half_items(const double (&qr)[NI], const double (&qi)[NI], const double (&pr)[NI],
+                                           const double (&pi)[NI], double yr, double yi, double (&Pr)[NP],
+                                           double (&Pi)[NP], double& ar, double& ai) {
+#pragma unroll
+    for (int p = HI - 1; p >= LO; --p) {
+        // below p: pr (the prefix); above p: already in y.  The first item's factor above is its neighbour times y
+        const bool single = p >= NP;
+        double& tr = single ? ar : Pr[p < NP ? p : 0];
+        double& ti = single ? ai : Pi[p < NP ? p : 0];
+        if (p > LO) {
+            if (FIRST && !single) cacc<true>(pr[p], pi[p], yr, yi, tr, ti);
+            else cacc<false>(pr[p], pi[p], yr, yi, tr, ti);
+            if (p > LO + 1) cmul_by(yr, yi, qr[p], qi[p]);
+        } else if (HI - LO > 1) {
+            if (FIRST && !single) cacc<true>(qr[LO + 1], qi[LO + 1], yr, yi, tr, ti);
+            else cacc<false>(qr[LO + 1], qi[LO + 1], yr, yi, tr, ti);
+        } else if (FIRST && !single) {
+            tr = yr;
+            ti = yi;
+        } else {
+            tr += yr;
+            ti += yi;
+        }
+    }
+}
+
+// One term: P[p] += w prod of the other items (FIRST: P[p] = ...), over the lane's items.  The thread's NI items
+// are two halves whose prefix and suffix chains run side by side (two complex chains keep the FP64 pipe busy
+// where one leaves it waiting), at the same number of multiplications as one chain.  The single item of an odd
+// column count is item NI - 1 and accumulates straight into its cofactor.
+template <int NP, bool ODD, int TPL, bool FIRST>
+__device__ __forceinline__ void pair_term(const double (&qr)[NP + ODD], const double (&qi)[NP + ODD], double w,
+                                          double (&Pr)[NP], double (&Pi)[NP], double& ar, double& ai) {
+    constexpr int NI = NP + ODD, NA = NI > 2 ? (NI + 1) / 2 : NI;
+    double pr[NI], pi[NI];
+    double ur = qr[0], ui = qi[0], vr = qr[NA < NI ? NA : 0], vi = qi[NA < NI ? NA : 0];
+#pragma unroll
+    for (int p = 1; p < NA; ++p) {
+        pr[p] = ur;
+        pi[p] = ui;
+        cmul_by(ur, ui, qr[p], qi[p]);
+        if (NA + p < NI) {
+            pr[NA + p < NI ? NA + p : 0] = vr;
+            pi[NA + p < NI ? NA + p : 0] = vi;
+            cmul_by(vr, vi, qr[NA + p < NI ? NA + p : 0], qi[NA + p < NI ? NA + p : 0]);
+        }
+    }
+    double yr, yi;
+    if constexpr (NA < NI) {
+        double tr = ur, ti = ui;
+        cmul_by(tr, ti, vr, vi);
+        lane_others<TPL>(tr, ti, yr, yi);
+        yr *= w;
+        yi *= w;
+        cmul_by(vr, vi, yr, yi);
+        cmul_by(ur, ui, yr, yi);
+        half_items<NA, NI, NP, NI, FIRST>(qr, qi, pr, pi, ur, ui, Pr, Pi, ar, ai);
+        half_items<0, NA, NP, NI, FIRST>(qr, qi, pr, pi, vr, vi, Pr, Pi, ar, ai);
+    } else {
+        lane_others<TPL>(ur, ui, yr, yi);
+        yr *= w;
+        yi *= w;
+        half_items<0, NI, NP, NI, FIRST>(qr, qi, pr, pi, yr, yi, Pr, Pi, ar, ai);
+    }
+}
+
+// KH columns per thread, lanes of TPL threads (tier KP = KH TPL); the plan has pair digits.
+template <int KH, int TPL, class SM>
+__device__ __forceinline__ void sweep_pairs_f64(SM& sm) {
+    constexpr int NP = KH / 2, ODD = KH & 1, NI = NP + ODD;
+    const auto& pl = sm.plan;
+    const auto& pt = pair_tables(sm);
+    const int tid = threadIdx.x;
+    const int lanes = blockDim.x / TPL, lane = tid / TPL, h = tid % TPL, c0 = h * KH;
+    const int wl0 = (tid & ~31) / TPL;                     // first lane of this warp: its lanes walk in lockstep
+    const int K = pl.K, Lin = pl.Lin, Lmid = pl.Lmid, nin = pl.nin;
+    const int64_t H = pl.H;
+    double ar[KH], ai[KH], x1r[NP], x1i[NP], x2r[NP], x2i[NP];
+#pragma unroll
+    for (int j = 0; j < KH; ++j) { ar[j] = 0.0; ai[j] = 0.0; }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) { x1r[p] = 0.0; x1i[p] = 0.0; x2r[p] = 0.0; x2i[p] = 0.0; }
+    for (int64_t hw = sm.chunk * lanes + wl0; hw < H; hw += (int64_t)lanes * sm.lane_mult) {
+        double sr[KH], si[KH], Lur[NP], Lui[NP], Lvr[NP], Lvi[NP], wh;
+        int64_t hl = hw + (lane - wl0);
+        const bool live = hl < H;                          // a lane past the end repeats lane H - 1 at weight 0
+        if (!live) hl = H - 1;
+        const uint64_t hpack = lane_digits(pl, hl, &wh);
+        if (!live) wh = 0.0;
+        lane_sums<KH, TPL>(sm, h, false, 0, hl, hpack, sr, si);
+#pragma unroll
+        for (int j = 0; j < KH; ++j) if (c0 + j >= K) { sr[j] = 1.0; si[j] = 0.0; }
+        {
+            const double2* bu = &sm.B[pl.pu][h];
+            const double2* bv = &sm.B[pl.pv][h];
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                const int a = 2 * p, b = 2 * p + 1;
+                // L = -2 (s_a d_b + s_b d_a) + 4 d_a d_b = -2 (s_a d_b + (s_b - 2 d_b) d_a) for the row d of u or v
+                auto lin = [&](double2 da, double2 db, double& re, double& im) {
+                    const double tr = fma(-2.0, db.x, sr[b]), ti = fma(-2.0, db.y, si[b]);
+                    re = fma(sr[a], db.x, fma(-si[a], db.y, fma(tr, da.x, -(ti * da.y))));
+                    im = fma(sr[a], db.y, fma(si[a], db.x, fma(tr, da.y, ti * da.x)));
+                    re *= -2.0;
+                    im *= -2.0;
+                };
+                lin(bu[a * TPL], bu[b * TPL], Lur[p], Lui[p]);
+                lin(bv[a * TPL], bv[b * TPL], Lvr[p], Lvi[p]);
+                const double2 c = pt.C[2 * p * TPL + h];
+                Lvr[p] += c.x;                             // L_v + C: the step from (1, 0) to (1, 1)
+                Lvi[p] += c.y;
+            }
+        }
+        for (int pm = 0; pm < Lmid; ++pm) {
+            const double wmh = wh * sm.tab_wm[pm];
+            const bool fwd = !(pm & 1);
+            // the transition into the block's first term: the middle digit's (none at the lane's first term)
+            unsigned e = pm > 0 ? (unsigned)sm.tab_fm[pm] : 0u;
+            double f = pm > 0 ? ((e & 0x80u) ? -2.0 : 2.0) : 0.0;
+            int kd = pm > 0 ? nin + (int)(e & 63u) : 0;
+            for (int i = 0;;) {
+                const int t = fwd ? i : Lin - 1 - i;
+                const double2* b = &sm.B[kd][h];
+                const double2* g = &pt.G[kd][h];
+#pragma unroll
+                for (int j = 0; j < KH; ++j) { sr[j] = fma(f, b[j * TPL].x, sr[j]); si[j] = fma(f, b[j * TPL].y, si[j]); }
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    Lur[p] = fma(f, g[2 * p * TPL].x, Lur[p]);
+                    Lui[p] = fma(f, g[2 * p * TPL].y, Lui[p]);
+                    Lvr[p] = fma(f, g[(2 * p + 1) * TPL].x, Lvr[p]);
+                    Lvi[p] = fma(f, g[(2 * p + 1) * TPL].y, Lvi[p]);
+                }
+                const double w = wmh * sm.tab_w[t];
+                double qr[NI], qi[NI], Pr[NP], Pi[NP];
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    qr[p] = fma(sr[2 * p], sr[2 * p + 1], -(si[2 * p] * si[2 * p + 1]));
+                    qi[p] = fma(sr[2 * p], si[2 * p + 1], si[2 * p] * sr[2 * p + 1]);
+                }
+                if (ODD) { qr[NI - 1] = sr[KH - 1]; qi[NI - 1] = si[KH - 1]; }
+                pair_term<NP, ODD, TPL, true>(qr, qi, w, Pr, Pi, ar[KH - 1], ai[KH - 1]);              // (0, 0)
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    x1r[p] -= Pr[p];
+                    x1i[p] -= Pi[p];
+                    qr[p] += Lur[p];
+                    qi[p] += Lui[p];
+                }
+                if (ODD) {
+                    qr[NI - 1] = fma(-2.0, sm.B[pl.pu][(KH - 1) * TPL + h].x, qr[NI - 1]);
+                    qi[NI - 1] = fma(-2.0, sm.B[pl.pu][(KH - 1) * TPL + h].y, qi[NI - 1]);
+                }
+                pair_term<NP, ODD, TPL, false>(qr, qi, -w, Pr, Pi, ar[KH - 1], ai[KH - 1]);            // (1, 0)
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    x2r[p] -= Pr[p];
+                    x2i[p] -= Pi[p];
+                    qr[p] += Lvr[p];
+                    qi[p] += Lvi[p];
+                }
+                if (ODD) {
+                    qr[NI - 1] = fma(-2.0, sm.B[pl.pv][(KH - 1) * TPL + h].x, qr[NI - 1]);
+                    qi[NI - 1] = fma(-2.0, sm.B[pl.pv][(KH - 1) * TPL + h].y, qi[NI - 1]);
+                }
+                pair_term<NP, ODD, TPL, false>(qr, qi, w, Pr, Pi, ar[KH - 1], ai[KH - 1]);             // (1, 1)
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    const double2 c = pt.C[2 * p * TPL + h];
+                    x1r[p] += Pr[p];
+                    x1i[p] += Pi[p];
+                    qr[p] -= Lur[p] + c.x;
+                    qi[p] -= Lui[p] + c.y;
+                }
+                if (ODD) {
+                    qr[NI - 1] = fma(2.0, sm.B[pl.pu][(KH - 1) * TPL + h].x, qr[NI - 1]);
+                    qi[NI - 1] = fma(2.0, sm.B[pl.pu][(KH - 1) * TPL + h].y, qi[NI - 1]);
+                }
+                pair_term<NP, ODD, TPL, false>(qr, qi, -w, Pr, Pi, ar[KH - 1], ai[KH - 1]);            // (0, 1)
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    x2r[p] += Pr[p];
+                    x2i[p] += Pi[p];
+                    const int a = 2 * p, c = 2 * p + 1;
+                    ar[a] = fma(Pr[p], sr[c], fma(-Pi[p], si[c], ar[a]));
+                    ai[a] = fma(Pr[p], si[c], fma(Pi[p], sr[c], ai[a]));
+                    ar[c] = fma(Pr[p], sr[a], fma(-Pi[p], si[a], ar[c]));
+                    ai[c] = fma(Pr[p], si[a], fma(Pi[p], sr[a], ai[c]));
+                }
+                if (++i == Lin) break;
+                e = sm.tab_f[fwd ? i : Lin - i];           // backward: the transition into t + 1, undone
+                kd = (int)(e & 63u);
+                f = (((e & 0x80u) != 0u) == fwd) ? -2.0 : 2.0;
+            }
+        }
+    }
+    {
+        const double2* bu = &sm.B[pl.pu][h];
+        const double2* bv = &sm.B[pl.pv][h];
+#pragma unroll
+        for (int j = 0; j < 2 * NP; ++j) {
+            const int p = j / 2;
+            const double2 du = bu[(j ^ 1) * TPL], dv = bv[(j ^ 1) * TPL];
+            const double tr = fma(du.x, x1r[p], fma(-du.y, x1i[p], fma(dv.x, x2r[p], -(dv.y * x2i[p]))));
+            const double ti = fma(du.x, x1i[p], fma(du.y, x1r[p], fma(dv.x, x2i[p], dv.y * x2r[p])));
+            ar[j] = fma(-2.0, tr, ar[j]);
+            ai[j] = fma(-2.0, ti, ai[j]);
+        }
+    }
+    reduce_to_P<KH, TPL>(ar, ai, sm, c0);
+}
+
+}  // namespace pe

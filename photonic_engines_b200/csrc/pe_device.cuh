@@ -80,18 +80,23 @@ struct PlanT {
     int Pin[NK];      // prefix products of the inner radices
     int Pmid[NK];     // prefix products of the middle radices
     unsigned char vend[NK];   // inner digit values after a forward inner block
+    int pairs;        // two digits are taken out of the walk as u, v of the pair sweep (fock_pairs.cuh)
+    int pu, pv;       // their kernel digits
     int sortR[NK];    // scratch of the planner: active digits by ascending radix
     int sortG[NK];
 };
 
+// Precision forms (the values of PE_PRECISION_* in pe_b200.h)
+constexpr int PREC_F64 = 0, PREC_MIXED = 1, PREC_COMP = 2;
+
 // Shared memory of one CTA working on one stream, for tiers of up to NK columns (32: the narrow layout
-// of chains up to 32 photons; 64: the wide one, FP64 only, so its FP32 copy of B is a placeholder).
-// COMP: the compensated form's layout, with the low parts of 2B beside the high ones.
-template <int NK, bool COMP = false>
+// of chains up to 32 photons; 64: the wide one, FP64 only).  Only the FP32 forms hold an FP32 copy of B, the
+// compensated one with its low parts beside the high ones.
+template <int NK, int PREC = PREC_F64>
 struct SmemT {
     static constexpr int NKMAX = NK;
-    static constexpr int NK32 = NK <= NARROW ? NK : 1;
-    static constexpr int NKLO = COMP ? NK32 : 1;
+    static constexpr int NK32 = PREC != PREC_F64 ? NK : 1;
+    static constexpr int NKLO = PREC == PREC_COMP ? NK32 : 1;
     PlanT<NK> plan;
     double2 P[NK];                 // cofactors of the step (scaled)
     double2 B[NK][NK];             // B[kd][j] = A[drow_kd, col_j], padded columns zero
@@ -114,26 +119,22 @@ struct SmemT {
     int gmul[NK];                // their multiplicities
     int ngrp;
     int64_t cur;                   // stream being processed (-1: queue drained)
-    int64_t lane0;                 // this CTA's first Gray lane (split steps: chunk * lanes)
+    int64_t chunk;                 // this CTA's chunk of the Gray lanes (split steps; 0 else)
     int lane_mult;                 // CTAs sharing one step of a stream (1 unless the step is split)
     double tot, target;
     int bad;                       // set by any thread that saw an out-of-range index
 };
 
-// Precision forms (the values of PE_PRECISION_* in pe_b200.h)
-constexpr int PREC_F64 = 0, PREC_MIXED = 1, PREC_COMP = 2;
-
-using Plan = PlanT<NARROW>;
-using Smem = SmemT<NARROW>;
 template <int KPM, int PREC = PREC_F64>
-using SmemFor = SmemT<(KPM <= NARROW ? NARROW : MAXN), PREC == PREC_COMP>;
+using SmemFor = SmemT<(KPM <= NARROW ? NARROW : MAXN), PREC>;
 
 // Dynamic shared memory of a chain CTA before its m weights: the layout of the tier, 16-byte rounded.
 template <int KPM, int PREC = PREC_F64>
 __host__ __device__ constexpr size_t smem_fixed_bytes() { return (sizeof(SmemFor<KPM, PREC>) + 15) & ~(size_t)15; }
 __host__ __device__ constexpr size_t smem_fixed_bytes_for(int kpm, int prec = PREC_F64) {
-    return kpm <= NARROW ? (prec == PREC_COMP ? smem_fixed_bytes<NARROW, PREC_COMP>() : smem_fixed_bytes<NARROW>())
-                         : smem_fixed_bytes<MAXN>();
+    return kpm > NARROW ? smem_fixed_bytes<MAXN>()
+         : prec == PREC_COMP ? smem_fixed_bytes<NARROW, PREC_COMP>()
+         : prec == PREC_MIXED ? smem_fixed_bytes<NARROW, PREC_MIXED>() : smem_fixed_bytes<NARROW>();
 }
 
 }  // namespace pe
