@@ -541,7 +541,7 @@ extern "C" int pe_cofactors_rows(int precision, const double* d_a, const int64_t
     const int kpm = kpm_for(K);
     if (kpm < 0) return PE_ERR_SIZE;
     if (kpm > NARROW && precision != PE_PRECISION_F64) return PE_ERR_SIZE;
-    if (tpl == 0) tpl = precision == PE_PRECISION_COMPENSATED ? default_tpl(kpm, precision) : (kpm <= 8 ? 1 : (kpm <= 40 ? 2 : 4));
+    if (tpl == 0) tpl = precision != PE_PRECISION_MIXED ? default_tpl(kpm, precision) : (kpm <= 8 ? 1 : 2);
     if (tpl_index(tpl) < 0) return PE_ERR_ARG;
     void* fn = find_cofactor_kernel(precision, tpl, kpm);
     if (!fn) return PE_ERR_SIZE;

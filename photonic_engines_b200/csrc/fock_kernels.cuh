@@ -125,15 +125,26 @@ static __device__ __forceinline__ void record_error(int* status, long long* deta
 }
 
 // ---------------------------------------------------------------------------------------- groups
-// Thread 0, after every pick: the distinct chosen modes and their multiplicities (the grouping of
+// One whole warp, after every pick: the distinct chosen modes and their multiplicities (the grouping of
 // cofactors_triton.py:419-427, kept incrementally instead of re-sorting the rows every step).
 template <class SM>
 __device__ __forceinline__ void add_to_groups(SM& sm, int row) {
-    for (int g = 0; g < sm.ngrp; ++g)
-        if (sm.grow[g] == row) { sm.gmul[g] += 1; return; }
-    sm.grow[sm.ngrp] = row;
-    sm.gmul[sm.ngrp] = 1;
-    sm.ngrp += 1;
+    const int lane = threadIdx.x & 31, D = sm.ngrp;
+    constexpr int GL = (SM::NKMAX + 31) / 32;
+    bool found = false;
+#pragma unroll
+    for (int q = 0; q < GL; ++q) {
+        const int g = lane + 32 * q;
+        const bool same = g < D && sm.grow[g < D ? g : 0] == row;
+        if (same) sm.gmul[g] += 1;
+        found = found || __any_sync(0xffffffffu, same);
+    }
+    if (!found && lane == 0) {
+        sm.grow[D] = row;
+        sm.gmul[D] = 1;
+        sm.ngrp = D + 1;
+    }
+    __syncwarp();
 }
 
 // One whole warp: the groups of sm.rows[0, count) (count <= 32) in order of first appearance, as
@@ -143,11 +154,9 @@ template <class SM>
 __device__ __forceinline__ void build_groups_warp(SM& sm, int count) {
     const int lane = threadIdx.x & 31;
     if (count > 32) {                                          // chains beyond 33 photons: serial
-        if (lane == 0) {
-            sm.ngrp = 0;
-            for (int i = 0; i < count; ++i) add_to_groups(sm, sm.rows[i]);
-        }
+        if (lane == 0) sm.ngrp = 0;
         __syncwarp();
+        for (int i = 0; i < count; ++i) add_to_groups(sm, sm.rows[i]);
         return;
     }
     const bool has = lane < count;
@@ -174,9 +183,9 @@ __device__ __forceinline__ T at_position(const T (&v)[GL], int p) {
     return __shfl_sync(0xffffffffu, x, p & 31);
 }
 
-// Exclusive prefix product over rank positions (position lane + 32 q in [q]), in place.
+// Inclusive prefix product over rank positions (position lane + 32 q in [q]), in place.
 template <int GL, typename T>
-__device__ __forceinline__ void exclusive_product(T (&v)[GL]) {
+__device__ __forceinline__ void inclusive_product(T (&v)[GL]) {
     const int lane = threadIdx.x & 31;
     T carry = T(1);
 #pragma unroll
@@ -187,12 +196,16 @@ __device__ __forceinline__ void exclusive_product(T (&v)[GL]) {
             const T y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x *= y;
         }
-        T ex = __shfl_up_sync(0xffffffffu, x, 1);
-        if (lane == 0) ex = T(1);
-        v[q] = ex * carry;
-        carry *= __shfl_sync(0xffffffffu, x, 31);
+        v[q] = x * carry;
+        if (q + 1 < GL) carry *= __shfl_sync(0xffffffffu, x, 31);
     }
 }
+
+// Terms of a step's sum: at most 2^31 before halving for 31 chosen rows, so 32 bits hold them in the narrow layouts.
+template <int NK> struct TermCount { typedef unsigned long long type; };
+template <> struct TermCount<8> { typedef unsigned type; };
+template <> struct TermCount<16> { typedef unsigned type; };
+template <> struct TermCount<32> { typedef unsigned type; };
 
 // Warp 0.  Lane g holds group g.  Radix = mult + 1, and one odd-multiplicity group (the last one)
 // has its radix halved to (mult + 1) / 2 with the scale doubled — the complement symmetry
@@ -200,8 +213,8 @@ __device__ __forceinline__ void exclusive_product(T (&v)[GL]) {
 // change N or the sum.  Active digits (radix >= 2) are ranked by ascending radix (then group); the
 // leading ones become the Gray lanes (best fill of the CTA's lanes), the next ones the inner block, then
 // the middle block; what does not fit the schedules joins the lanes.  The ranking takes one ballot per
-// distinct radix value, and every digit's table entries are written by the lane of its rank, so only
-// the choice of the three splits walks the ranks one by one (in registers, read by shuffles).
+// distinct radix value; the three splits are ballots over the ranks' prefix products (which only grow), and every
+// digit's table entries are written by the lane of its rank.
 // pair_lanes > 0: take two digits of multiplicity 1 out for the pair sweep of that many lanes, when there are
 // two; N then counts its blocks of four terms.
 template <class SM>
@@ -270,66 +283,81 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
         }
     }
     __syncwarp();
-    long long rv[GL];                                  // radix at rank position lane + 32 q (1 past na)
-#pragma unroll
-    for (int q = 0; q < GL; ++q) rv[q] = lane + 32 * q < na ? pl.sortR[lane + 32 * q] : 1;
-    long long pre[GL];                                 // product of the radices at positions <= p
-#pragma unroll
-    for (int q = 0; q < GL; ++q) pre[q] = rv[q];
-    exclusive_product<GL>(pre);
-#pragma unroll
-    for (int q = 0; q < GL; ++q) pre[q] *= rv[q];
-    const long long N = na > 0 ? at_position<GL>(pre, na - 1) : 1;
-    // lanes: the prefix of the ranked digits that best fills the CTA's lanes
-    int nhi = na;
-    if (N > lanes) {
-        double best = -1.0;
-        nhi = 1;
-        for (int i = 0; i < na; ++i) {
-            const long long prod = at_position<GL>(pre, i);
-            if (i > 0 && prod > N / 4) break;          // N / prod < 4
-            const double e = prod >= lanes
-                ? (double)prod / ((double)lanes * (double)((prod + lanes - 1) / lanes))
-                : (double)prod / (double)lanes;
-            if (e > best + 1e-12) { best = e; nhi = i + 1; }
-            if (prod >= lanes && e >= 0.95) break;
-        }
-    }
-    int nin = 0, Lin = 1;
-    while (nhi + nin < na) {
-        const int r = (int)at_position<GL>(rv, nhi + nin);
-        if (Lin * r > lin_max) break;
-        Lin *= r;
-        ++nin;
-    }
-    int nmid = 0, Lmid = 1;
-    while (nhi + nin + nmid < na) {
-        const int r = (int)at_position<GL>(rv, nhi + nin + nmid);
-        if (Lmid * r > mid_max) break;
-        Lmid *= r;
-        ++nmid;
-    }
-    // digit order: inner (kd 0..nin-1), middle, lanes, digits beyond both schedules (more lanes), then the
-    // fixed digits (radix 1) in group order; Pin / Pmid the prefix products of the inner / middle radices
-    int pin[GL], pmid[GL];
+    using TC = typename TermCount<SM::NKMAX>::type;
+    TC rv[GL], pre[GL];                                // radix at rank position lane + 32 q (1 past na), and the
+    int gp[GL], mp[GL];                                // product of the radices up to it; its group and multiplicity
 #pragma unroll
     for (int q = 0; q < GL; ++q) {
         const int p = lane + 32 * q;
-        pin[q] = (p >= nhi && p < nhi + nin) ? (int)rv[q] : 1;
-        pmid[q] = (p >= nhi + nin && p < nhi + nin + nmid) ? (int)rv[q] : 1;
+        rv[q] = p < na ? (TC)pl.sortR[p] : TC(1);
+        gp[q] = p < na ? pl.sortG[p] : 0;
+        mp[q] = p < na ? sm.gmul[gp[q]] : 1;
+        pre[q] = rv[q];
     }
-    exclusive_product<GL>(pin);
-    exclusive_product<GL>(pmid);
+    inclusive_product<GL>(pre);
+    const TC N = na > 0 ? at_position<GL>(pre, na - 1) : TC(1);
+    // lanes: the prefix of the ranked digits that best fills the CTA's lanes and leaves every lane four terms; the
+    // first that fills 95 % of them, else the fullest
+    int nhi = na;
+    if (N > (TC)lanes) {
+        unsigned fill[GL];
+        int stop = 64;
+#pragma unroll
+        for (int q = 0; q < GL; ++q) {
+            const int p = lane + 32 * q;
+            const bool ok = p < na && (p == 0 || pre[q] <= N / 4);
+            const TC rounds = pre[q] >= (TC)lanes ? (pre[q] + (TC)lanes - 1) / (TC)lanes : TC(1);
+            const float e = (float)pre[q] / ((float)lanes * (float)rounds);
+            fill[q] = ok ? __float_as_uint(e) : 0u;
+            const unsigned full95 = __ballot_sync(full, ok && pre[q] >= (TC)lanes && e >= 0.95f);
+            if (full95 && stop == 64) stop = 32 * q + __ffs(full95) - 1;
+        }
+        unsigned best = 0u;
+#pragma unroll
+        for (int q = 0; q < GL; ++q) {
+            if (lane + 32 * q > stop) fill[q] = 0u;
+            best = max(best, __reduce_max_sync(full, fill[q]));
+        }
+        nhi = 0;
+#pragma unroll
+        for (int q = 0; q < GL; ++q) {
+            const unsigned at = __ballot_sync(full, fill[q] == best);
+            if (at && nhi == 0) nhi = 32 * q + __ffs(at);
+        }
+    }
+    // the digits p >= p0 whose product from p0 on stays within lim: how many, their product, and (own position)
+    // the product of those below it
+    const TC ph = nhi > 0 ? at_position<GL>(pre, nhi - 1) : TC(1);
+    int pin[GL], pmid[GL];
+    bool ones_in = true, ones_mid = true;              // schedules of digits of multiplicity 1 only
+    auto block = [&](int p0, TC base, int lim, int (&ex)[GL], bool& ones, int& L) {
+        int n = 0;
+#pragma unroll
+        for (int q = 0; q < GL; ++q) {
+            const int p = lane + 32 * q;
+            const TC from = p >= p0 && p < na ? pre[q] / base : TC(0);
+            const bool in = from > 0 && from <= (TC)lim;
+            ex[q] = in ? (int)(from / rv[q]) : 1;
+            n += __popc(__ballot_sync(full, in));
+            ones = __all_sync(full, !in || (rv[q] == 2 && mp[q] == 1)) && ones;
+        }
+        L = n > 0 ? (int)(at_position<GL>(pre, p0 + n - 1) / base) : 1;
+        return n;
+    };
+    int Lin, Lmid;
+    const int nin = block(nhi, ph, lin_max, pin, ones_in, Lin);
+    const int nmid = block(nhi + nin, ph * (TC)Lin, mid_max, pmid, ones_mid, Lmid);
+    // digit order: inner (kd 0..nin-1), middle, lanes, digits beyond both schedules (more lanes), then the
+    // fixed digits (radix 1) in group order; Pin / Pmid the prefix products of the inner / middle radices
     int nfix = 0;
 #pragma unroll
     for (int q = 0; q < GL; ++q) {
         const int p = lane + 32 * q;
         if (p < na) {
-            const int g = pl.sortG[p];
             const int kd = p < nhi ? nin + nmid + p : (p < nhi + nin + nmid ? p - nhi : p);
             pl.R[kd] = (int)rv[q];
-            pl.M[kd] = sm.gmul[g];
-            pl.drow[kd] = sm.grow[g];
+            pl.M[kd] = mp[q];
+            pl.drow[kd] = sm.grow[gp[q]];
             if (p >= nhi && p < nhi + nin) pl.Pin[kd] = pin[q];
             if (p >= nhi + nin && p < nhi + nin + nmid) pl.Pmid[kd - nin] = pmid[q];
         }
@@ -351,34 +379,31 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
         pl.drow[kd] = sm.grow[lane == 0 ? gu : gv];
     }
     if (lane == 0) {
+        pl.ones_in = ones_in; pl.ones_mid = ones_mid;
         pl.pairs = gv >= 0;
         pl.pu = na + nfix;
         pl.pv = na + nfix + 1;
-        pl.N = N; pl.H = N / ((long long)Lin * Lmid); pl.Lin = Lin; pl.Lmid = Lmid;
+        pl.N = (int64_t)N; pl.H = (int64_t)(N / ((TC)Lin * (TC)Lmid)); pl.Lin = Lin; pl.Lmid = Lmid;
         pl.K = K; pl.K1 = K1; pl.D = D;
         pl.nin = nin; pl.nmid = nmid; pl.nhi = na - nin - nmid;
         pl.scale = (halved >= 0 ? 2.0 : 1.0) * ldexp(1.0, -K1);
     }
 }
 
+// Entry t of a reflected Gray schedule over the nd digits from d0 on (prefix products Pp): the digit that moves
+// into t (| 0x80 when it moves up: the column sums then move by -2 b), and the weight prod (-1)^v C(M, v) at t.
+// ones: every digit has radix 2 and multiplicity 1, so the digits are the bits of the Gray code of t and the
+// weight its parity.  vend (optional): the digit values at t.
 template <class PL>
 static __device__ __forceinline__ unsigned char gray_entry(const PL& pl, int d0, int nd, const int* Pp, int t,
-                                                          double* w_out, unsigned char* vend, bool binary) {
-    if (binary) {                                   // every radix 2: the digits are the bits of t
-        const int qstar = t > 0 ? __ffs(t) - 1 : -1;
-        int par = 0, parh = 0;
-        double w = 1.0;
-        for (int q = nd - 1; q >= 0; --q) {
-            if (q == qstar) parh = par;
-            const int d = (t >> q) & 1;
-            const int v = (par & 1) ? 1 - d : d;
-            if (vend) vend[q] = (unsigned char)v;
-            par += v;
-            if (v) w *= -(double)pl.M[d0 + q];      // (-1)^v C(M, v) at v = 1
-        }
-        *w_out = w;
-        if (qstar < 0) return 0;
-        return (unsigned char)(qstar | ((parh & 1) ? 0 : 0x80));
+                                                          double* w_out, unsigned char* vend, bool ones) {
+    if (ones) {
+        const int g = t ^ (t >> 1);
+        if (vend) for (int q = 0; q < nd; ++q) vend[q] = (unsigned char)((g >> q) & 1);
+        *w_out = (t & 1) ? -1.0 : 1.0;
+        if (t == 0) return 0;
+        const int q = __ffs(t) - 1;
+        return (unsigned char)(q | (((g >> q) & 1) ? 0x80 : 0));
     }
     int qstar = -1;
     if (t > 0) {
@@ -390,11 +415,11 @@ static __device__ __forceinline__ unsigned char gray_entry(const PL& pl, int d0,
     for (int q = nd - 1; q >= 0; --q) {
         if (q == qstar) parh = par;
         const int R = pl.R[d0 + q];
-        const int d = (t / Pp[q]) % R;
+        const int d = R == 2 ? (t / Pp[q]) & 1 : (t / Pp[q]) % R;
         const int v = (par & 1) ? R - 1 - d : d;
         if (vend) vend[q] = (unsigned char)v;
         par += v;
-        w *= signed_binom(pl.M[d0 + q], v);
+        if (v) w *= signed_binom(pl.M[d0 + q], v);
     }
     *w_out = w;
     if (qstar < 0) return 0;
@@ -452,18 +477,15 @@ static __device__ void prepare_step(SM& sm, const double2* __restrict__ A, int64
                 make_float4((float)(2.0 * b1.x), (float)(2.0 * b2.x), (float)(2.0 * b1.y), (float)(2.0 * b2.y));
         }
     }
-    bool bin_in = true, bin_mid = true;             // schedules of radix-2 digits only (distinct rows)
-    for (int q = 0; q < pl.nin; ++q) bin_in = bin_in && pl.R[q] == 2;
-    for (int q = 0; q < pl.nmid; ++q) bin_mid = bin_mid && pl.R[pl.nin + q] == 2;
     for (int t = tid; t < pl.Lin; t += T) {
         double w;
-        sm.tab_f[t] = gray_entry(pl, 0, pl.nin, pl.Pin, t, &w, t == pl.Lin - 1 ? sm.plan.vend : nullptr, bin_in);
+        sm.tab_f[t] = gray_entry(pl, 0, pl.nin, pl.Pin, t, &w, t == pl.Lin - 1 ? sm.plan.vend : nullptr, pl.ones_in);
         sm.tab_w[t] = w;
         sm.tab_w32[t] = (float)w;
     }
     for (int t = tid; t < pl.Lmid; t += T) {
         double w;
-        sm.tab_fm[t] = gray_entry(pl, pl.nin, pl.nmid, pl.Pmid, t, &w, nullptr, bin_mid);
+        sm.tab_fm[t] = gray_entry(pl, pl.nin, pl.nmid, pl.Pmid, t, &w, nullptr, pl.ones_mid);
         sm.tab_wm[t] = w;
     }
 }
@@ -1127,22 +1149,22 @@ __device__ __forceinline__ void cofactor_step(SM& sm, const double2* A, int64_t 
 // ---------------------------------------------------------------------------------------- draw
 // Marginal over the m output modes, FP64 block scan (contiguous chunk per thread, warp scan, warps
 // in order), then idx = min(#{rho : cw_rho < u * tot}, m - 1) with tot = cw[m - 1]
-// (cofactors_triton.py:298-308).  Thread 0 records the pick and updates the groups; the gap
+// (cofactors_triton.py:298-308).  Warp 0 records the pick and updates the groups; the gap
 // min |cw - u tot| / tot is left in sm.fmin[0].
 template <class SM>
 static __device__ void draw_step(SM& sm, double* __restrict__ wgt, const double2* __restrict__ A, int64_t rs, int64_t cs,
                                  int m, int k, double u, double* __restrict__ marg_row, bool update_groups) {
     const int tid = threadIdx.x, T = blockDim.x, lid = tid & 31, wid = tid >> 5, nw = T >> 5;
-    // DR modes per thread at a time, and the column loop unrolled 4 times, so that 16 independent loads of
+    // DR modes per thread at a time, and the column loop unrolled DC times, so that 16 or 32 independent loads of
     // A (from L2) are in flight instead of one; the sum over columns keeps its order (same bits as one mode
     // at a time).  The draw is bound by L2 latency, not by its few FLOPs (m = 900, the c3 batch: 4-5 %
     // faster than two columns ahead).
-    constexpr int DR = 4;
+    constexpr int DR = 4, DC = PE_MAXT * PE_MINB <= 256 ? 8 : 4;      // as many as the kernel's registers hold
     for (int rho0 = tid; rho0 < m; rho0 += T * DR) {
         double xr[DR], xi[DR];
 #pragma unroll
         for (int r = 0; r < DR; ++r) { xr[r] = 0.0; xi[r] = 0.0; }
-#pragma unroll 4
+#pragma unroll DC
         for (int c = 0; c < k; ++c) {
             const int64_t co = (int64_t)sm.cols[c] * cs;
             const double2 p = sm.P[c];
@@ -1210,13 +1232,17 @@ static __device__ void draw_step(SM& sm, double* __restrict__ wgt, const double2
     }
     if (lid == 0) { sm.cnt[wid] = cnt; sm.fmin[wid] = gmin; }
     __syncthreads();
-    if (tid == 0) {
-        int c = 0;
-        double g = 1.0e300;
-        for (int w = 0; w < nw; ++w) { c += sm.cnt[w]; g = fmin(g, sm.fmin[w]); }
+    if (wid == 0) {
+        int c = lid < nw ? sm.cnt[lid] : 0;
+        double g = lid < nw ? sm.fmin[lid] : 1.0e300;
+        c = __reduce_add_sync(0xffffffffu, c);
+#pragma unroll
+        for (int o = MAX_WARPS / 2; o > 0; o >>= 1) g = fmin(g, __shfl_xor_sync(0xffffffffu, g, o));
         const int pick = min(c, m - 1);
-        sm.rows[k - 1] = pick;
-        sm.fmin[0] = g / tot;
+        if (lid == 0) {
+            sm.rows[k - 1] = pick;
+            sm.fmin[0] = g / tot;
+        }
         if (update_groups) add_to_groups(sm, pick);
     }
     __syncthreads();
@@ -1245,6 +1271,15 @@ __device__ void chain_one(const ChainParams& p, SmemFor<KPM, PREC>& sm, double* 
         if (r < 0 || r >= m) atomicOr(&sm.bad, 1);
         else sm.rows[tid] = (int)r;
     }
+    if (ok && tid >= kf - 1 && tid < nk) {                     // every step's uniform at once, one step per thread
+        if (p.uniforms) {
+            sm.u[tid] = p.uniforms[s * p.n_stride + tid];
+        } else {
+            const int64_t row = p.seed_row ? p.seed_row[s] : 0;
+            const int64_t ro = p.rng_off ? p.rng_off[s] : s;
+            sm.u[tid] = chain_uniform((uint64_t)p.seeds[row * p.n_stride + tid], ro);
+        }
+    }
     if (!ok && tid == 0) sm.bad = 1;
     if (tid == 0) { sm.ngrp = 0; sm.chunk = 0; sm.lane_mult = 1; }
     __syncthreads();
@@ -1266,14 +1301,7 @@ __device__ void chain_one(const ChainParams& p, SmemFor<KPM, PREC>& sm, double* 
         } else {
             cofactor_step<TPL, KPM, PREC>(sm, A, 1, m, K1, K);
         }
-        double u;
-        if (p.uniforms) {
-            u = p.uniforms[s * p.n_stride + (k - 1)];
-        } else {
-            const int64_t row = p.seed_row ? p.seed_row[s] : 0;
-            const int64_t ro = p.rng_off ? p.rng_off[s] : s;
-            u = chain_uniform((uint64_t)p.seeds[row * p.n_stride + (k - 1)], ro);
-        }
+        const double u = sm.u[k - 1];
         double* mrow = p.marg ? p.marg + ((size_t)s * p.n_stride + (k - 1)) * p.marg_stride : nullptr;
         if constexpr (PREC != PREC_F64) {
             draw_step(sm, wgt, A, 1, m, m, k, u, mrow, false);
@@ -1281,7 +1309,7 @@ __device__ void chain_one(const ChainParams& p, SmemFor<KPM, PREC>& sm, double* 
                 dispatch_f64<4, KPM>(sm, K);
                 draw_step(sm, wgt, A, 1, m, m, k, u, mrow, false);
             }
-            if (tid == 0) add_to_groups(sm, sm.rows[k - 1]);
+            if (tid < 32) add_to_groups(sm, sm.rows[k - 1]);
             __syncthreads();
         } else {
             draw_step(sm, wgt, A, 1, m, m, k, u, mrow, true);

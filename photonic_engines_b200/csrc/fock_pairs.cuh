@@ -72,6 +72,17 @@ static __device__ void prepare_pairs(SM& sm, int kh, int tl) {
     }
 }
 
+// The sweep's values: double (FP64 form), or float2 (plain mixed form: two column groups of a thread side by side on
+// paired FP32 instructions).
+__device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ double vmul(double a, double b) { return a * b; }
+__device__ __forceinline__ double vadd(double a, double b) { return a + b; }
+__device__ __forceinline__ double vneg(double a) { return -a; }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
+
 // The product of the other threads' totals of a lane (TPL 2: the partner's; TPL 4: two butterfly exchanges).
 template <int TPL>
 __device__ __forceinline__ void lane_others(double xr, double xi, double& yr, double& yi) {
@@ -90,36 +101,51 @@ __device__ __forceinline__ void lane_others(double xr, double xi, double& yr, do
     }
 }
 
-// P (+)= x y, complex (FIRST: P = x y).
-template <bool FIRST>
-__device__ __forceinline__ void cacc(double xr, double xi, double yr, double yi, double& Pr, double& Pi) {
-    if (FIRST) {
-        Pr = fma(xr, yr, -(xi * yi));
-        Pi = fma(xr, yi, xi * yr);
-    } else {
-        Pr = fma(xr, yr, Pr);
-        Pr = fma(-xi, yi, Pr);
-        Pi = fma(xr, yi, Pi);
-        Pi = fma(xi, yr, Pi);
+// The same for paired values, each half counting as a thread of its own.
+template <int TPL>
+__device__ __forceinline__ void lane_others(float2 xr, float2 xi, float2& yr, float2& yi) {
+    yr = make_float2(xr.y, xr.x);
+    yi = make_float2(xi.y, xi.x);
+    if constexpr (TPL == 2) {
+        const float tr = fmaf(xr.x, xr.y, -(xi.x * xi.y)), ti = fmaf(xr.x, xi.y, xi.x * xr.y);
+        const float Tr = __shfl_xor_sync(0xffffffffu, tr, 1), Ti = __shfl_xor_sync(0xffffffffu, ti, 1);
+        const float2 R = make_float2(Tr, Tr), I = make_float2(Ti, Ti);
+        const float2 nr = vfma(yr, R, vneg(vmul(yi, I)));
+        yi = vfma(yr, I, vmul(yi, R));
+        yr = nr;
     }
 }
-__device__ __forceinline__ void cmul_by(double& xr, double& xi, double yr, double yi) {
-    const double nr = fma(xr, yr, -(xi * yi));
-    xi = fma(xr, yi, xi * yr);
+
+// P (+)= x y, complex (FIRST: P = x y).
+template <bool FIRST, typename V>
+__device__ __forceinline__ void cacc(V xr, V xi, V yr, V yi, V& Pr, V& Pi) {
+    if (FIRST) {
+        Pr = vfma(xr, yr, vneg(vmul(xi, yi)));
+        Pi = vfma(xr, yi, vmul(xi, yr));
+    } else {
+        Pr = vfma(xr, yr, Pr);
+        Pr = vfma(vneg(xi), yi, Pr);
+        Pi = vfma(xr, yi, Pi);
+        Pi = vfma(xi, yr, Pi);
+    }
+}
+template <typename V>
+__device__ __forceinline__ void cmul_by(V& xr, V& xi, V yr, V yi) {
+    const V nr = vfma(xr, yr, vneg(vmul(xi, yi)));
+    xi = vfma(xr, yi, vmul(xi, yr));
     xr = nr;
 }
 
 // The items [LO, HI) of one half, y = the product of everything else: P[p] += y prod of the half's other items.
-template <int LO, int HI, int NP, int NI, bool FIRST>
-__device__ __forceinline__ void half_items(const double (&qr)[NI], const double (&qi)[NI], const double (&pr)[NI],
-                                           const double (&pi)[NI], double yr, double yi, double (&Pr)[NP],
-                                           double (&Pi)[NP], double& ar, double& ai) {
+template <int LO, int HI, int NP, int NI, bool FIRST, typename V>
+__device__ __forceinline__ void half_items(const V (&qr)[NI], const V (&qi)[NI], const V (&pr)[NI], const V (&pi)[NI],
+                                           V yr, V yi, V (&Pr)[NP], V (&Pi)[NP], V& ar, V& ai) {
 #pragma unroll
     for (int p = HI - 1; p >= LO; --p) {
         // below p: pr (the prefix); above p: already in y.  The first item's factor above is its neighbour times y
         const bool single = p >= NP;
-        double& tr = single ? ar : Pr[p < NP ? p : 0];
-        double& ti = single ? ai : Pi[p < NP ? p : 0];
+        V& tr = single ? ar : Pr[p < NP ? p : 0];
+        V& ti = single ? ai : Pi[p < NP ? p : 0];
         if (p > LO) {
             if (FIRST && !single) cacc<true>(pr[p], pi[p], yr, yi, tr, ti);
             else cacc<false>(pr[p], pi[p], yr, yi, tr, ti);
@@ -131,8 +157,8 @@ __device__ __forceinline__ void half_items(const double (&qr)[NI], const double 
             tr = yr;
             ti = yi;
         } else {
-            tr += yr;
-            ti += yi;
+            tr = vadd(tr, yr);
+            ti = vadd(ti, yi);
         }
     }
 }
@@ -141,12 +167,12 @@ __device__ __forceinline__ void half_items(const double (&qr)[NI], const double 
 // are two halves whose prefix and suffix chains run side by side (two complex chains keep the FP64 pipe busy
 // where one leaves it waiting), at the same number of multiplications as one chain.  The single item of an odd
 // column count is item NI - 1 and accumulates straight into its cofactor.
-template <int NP, bool ODD, int TPL, bool FIRST>
-__device__ __forceinline__ void pair_term(const double (&qr)[NP + ODD], const double (&qi)[NP + ODD], double w,
-                                          double (&Pr)[NP], double (&Pi)[NP], double& ar, double& ai) {
+template <int NP, bool ODD, int TPL, bool FIRST, typename V>
+__device__ __forceinline__ void pair_term(const V (&qr)[NP + ODD], const V (&qi)[NP + ODD], V w, V (&Pr)[NP],
+                                          V (&Pi)[NP], V& ar, V& ai) {
     constexpr int NI = NP + ODD, NA = NI > 2 ? (NI + 1) / 2 : NI;
-    double pr[NI], pi[NI];
-    double ur = qr[0], ui = qi[0], vr = qr[NA < NI ? NA : 0], vi = qi[NA < NI ? NA : 0];
+    V pr[NI], pi[NI];
+    V ur = qr[0], ui = qi[0], vr = qr[NA < NI ? NA : 0], vi = qi[NA < NI ? NA : 0];
 #pragma unroll
     for (int p = 1; p < NA; ++p) {
         pr[p] = ur;
@@ -158,29 +184,98 @@ __device__ __forceinline__ void pair_term(const double (&qr)[NP + ODD], const do
             cmul_by(vr, vi, qr[NA + p < NI ? NA + p : 0], qi[NA + p < NI ? NA + p : 0]);
         }
     }
-    double yr, yi;
+    V yr, yi;
     if constexpr (NA < NI) {
-        double tr = ur, ti = ui;
+        V tr = ur, ti = ui;
         cmul_by(tr, ti, vr, vi);
         lane_others<TPL>(tr, ti, yr, yi);
-        yr *= w;
-        yi *= w;
+        yr = vmul(yr, w);
+        yi = vmul(yi, w);
         cmul_by(vr, vi, yr, yi);
         cmul_by(ur, ui, yr, yi);
-        half_items<NA, NI, NP, NI, FIRST>(qr, qi, pr, pi, ur, ui, Pr, Pi, ar, ai);
-        half_items<0, NA, NP, NI, FIRST>(qr, qi, pr, pi, vr, vi, Pr, Pi, ar, ai);
+        half_items<NA, NI, NP, NI, FIRST, V>(qr, qi, pr, pi, ur, ui, Pr, Pi, ar, ai);
+        half_items<0, NA, NP, NI, FIRST, V>(qr, qi, pr, pi, vr, vi, Pr, Pi, ar, ai);
     } else {
         lane_others<TPL>(ur, ui, yr, yi);
-        yr *= w;
-        yi *= w;
-        half_items<0, NI, NP, NI, FIRST>(qr, qi, pr, pi, yr, yi, Pr, Pi, ar, ai);
+        yr = vmul(yr, w);
+        yi = vmul(yi, w);
+        half_items<0, NI, NP, NI, FIRST, V>(qr, qi, pr, pi, yr, yi, Pr, Pi, ar, ai);
+    }
+}
+
+// The four terms of one block from the column sums s at u = v = 0 and the walked L_u, L_v + C: products of the
+// pairs, all-but-one sums P, and their shares of the cofactors (a) and of X_u, X_v (x1, x2).  getc(p): C of pair p;
+// getd(d): step of the single column's sum when u (d = 0) or v (d = 1) moves to 1.
+template <int KH, int TPL, typename V, class GetC, class GetD>
+__device__ __forceinline__ void pair_block(const V (&sr)[KH], const V (&si)[KH], const V (&Lur)[KH / 2],
+                                           const V (&Lui)[KH / 2], const V (&Lvr)[KH / 2], const V (&Lvi)[KH / 2], V w,
+                                           V (&ar)[KH], V (&ai)[KH], V (&x1r)[KH / 2], V (&x1i)[KH / 2],
+                                           V (&x2r)[KH / 2], V (&x2i)[KH / 2], GetC getc, GetD getd) {
+    constexpr int NP = KH / 2, ODD = KH & 1, NI = NP + ODD;
+    V qr[NI], qi[NI], Pr[NP], Pi[NP], cr, ci;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        qr[p] = vfma(sr[2 * p], sr[2 * p + 1], vneg(vmul(si[2 * p], si[2 * p + 1])));
+        qi[p] = vfma(sr[2 * p], si[2 * p + 1], vmul(si[2 * p], sr[2 * p + 1]));
+    }
+    if (ODD) { qr[NI - 1] = sr[KH - 1]; qi[NI - 1] = si[KH - 1]; }
+    pair_term<NP, ODD, TPL, true, V>(qr, qi, w, Pr, Pi, ar[KH - 1], ai[KH - 1]);                // (0, 0)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        x1r[p] = vadd(x1r[p], vneg(Pr[p]));
+        x1i[p] = vadd(x1i[p], vneg(Pi[p]));
+        qr[p] = vadd(qr[p], Lur[p]);
+        qi[p] = vadd(qi[p], Lui[p]);
+    }
+    if (ODD) {
+        getd(0, cr, ci);
+        qr[NI - 1] = vadd(qr[NI - 1], cr);
+        qi[NI - 1] = vadd(qi[NI - 1], ci);
+    }
+    pair_term<NP, ODD, TPL, false, V>(qr, qi, vneg(w), Pr, Pi, ar[KH - 1], ai[KH - 1]);         // (1, 0)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        x2r[p] = vadd(x2r[p], vneg(Pr[p]));
+        x2i[p] = vadd(x2i[p], vneg(Pi[p]));
+        qr[p] = vadd(qr[p], Lvr[p]);
+        qi[p] = vadd(qi[p], Lvi[p]);
+    }
+    if (ODD) {
+        getd(1, cr, ci);
+        qr[NI - 1] = vadd(qr[NI - 1], cr);
+        qi[NI - 1] = vadd(qi[NI - 1], ci);
+    }
+    pair_term<NP, ODD, TPL, false, V>(qr, qi, w, Pr, Pi, ar[KH - 1], ai[KH - 1]);               // (1, 1)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        getc(p, cr, ci);
+        x1r[p] = vadd(x1r[p], Pr[p]);
+        x1i[p] = vadd(x1i[p], Pi[p]);
+        qr[p] = vadd(qr[p], vneg(vadd(Lur[p], cr)));
+        qi[p] = vadd(qi[p], vneg(vadd(Lui[p], ci)));
+    }
+    if (ODD) {
+        getd(0, cr, ci);
+        qr[NI - 1] = vadd(qr[NI - 1], vneg(cr));
+        qi[NI - 1] = vadd(qi[NI - 1], vneg(ci));
+    }
+    pair_term<NP, ODD, TPL, false, V>(qr, qi, vneg(w), Pr, Pi, ar[KH - 1], ai[KH - 1]);         // (0, 1)
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        x2r[p] = vadd(x2r[p], Pr[p]);
+        x2i[p] = vadd(x2i[p], Pi[p]);
+        const int a = 2 * p, b = 2 * p + 1;
+        ar[a] = vfma(Pr[p], sr[b], vfma(vneg(Pi[p]), si[b], ar[a]));
+        ai[a] = vfma(Pr[p], si[b], vfma(Pi[p], sr[b], ai[a]));
+        ar[b] = vfma(Pr[p], sr[a], vfma(vneg(Pi[p]), si[a], ar[b]));
+        ai[b] = vfma(Pr[p], si[a], vfma(Pi[p], sr[a], ai[b]));
     }
 }
 
 // KH columns per thread, lanes of TPL threads (tier KP = KH TPL); the plan has pair digits.
 template <int KH, int TPL, class SM>
 __device__ __forceinline__ void sweep_pairs_f64(SM& sm) {
-    constexpr int NP = KH / 2, ODD = KH & 1, NI = NP + ODD;
+    constexpr int NP = KH / 2;
     const auto& pl = sm.plan;
     const auto& pt = pair_tables(sm);
     const int tid = threadIdx.x;
@@ -245,61 +340,18 @@ __device__ __forceinline__ void sweep_pairs_f64(SM& sm) {
                     Lvi[p] = fma(f, g[(2 * p + 1) * TPL].y, Lvi[p]);
                 }
                 const double w = wmh * sm.tab_w[t];
-                double qr[NI], qi[NI], Pr[NP], Pi[NP];
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    qr[p] = fma(sr[2 * p], sr[2 * p + 1], -(si[2 * p] * si[2 * p + 1]));
-                    qi[p] = fma(sr[2 * p], si[2 * p + 1], si[2 * p] * sr[2 * p + 1]);
-                }
-                if (ODD) { qr[NI - 1] = sr[KH - 1]; qi[NI - 1] = si[KH - 1]; }
-                pair_term<NP, ODD, TPL, true>(qr, qi, w, Pr, Pi, ar[KH - 1], ai[KH - 1]);              // (0, 0)
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    x1r[p] -= Pr[p];
-                    x1i[p] -= Pi[p];
-                    qr[p] += Lur[p];
-                    qi[p] += Lui[p];
-                }
-                if (ODD) {
-                    qr[NI - 1] = fma(-2.0, sm.B[pl.pu][(KH - 1) * TPL + h].x, qr[NI - 1]);
-                    qi[NI - 1] = fma(-2.0, sm.B[pl.pu][(KH - 1) * TPL + h].y, qi[NI - 1]);
-                }
-                pair_term<NP, ODD, TPL, false>(qr, qi, -w, Pr, Pi, ar[KH - 1], ai[KH - 1]);            // (1, 0)
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    x2r[p] -= Pr[p];
-                    x2i[p] -= Pi[p];
-                    qr[p] += Lvr[p];
-                    qi[p] += Lvi[p];
-                }
-                if (ODD) {
-                    qr[NI - 1] = fma(-2.0, sm.B[pl.pv][(KH - 1) * TPL + h].x, qr[NI - 1]);
-                    qi[NI - 1] = fma(-2.0, sm.B[pl.pv][(KH - 1) * TPL + h].y, qi[NI - 1]);
-                }
-                pair_term<NP, ODD, TPL, false>(qr, qi, w, Pr, Pi, ar[KH - 1], ai[KH - 1]);             // (1, 1)
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    const double2 c = pt.C[2 * p * TPL + h];
-                    x1r[p] += Pr[p];
-                    x1i[p] += Pi[p];
-                    qr[p] -= Lur[p] + c.x;
-                    qi[p] -= Lui[p] + c.y;
-                }
-                if (ODD) {
-                    qr[NI - 1] = fma(2.0, sm.B[pl.pu][(KH - 1) * TPL + h].x, qr[NI - 1]);
-                    qi[NI - 1] = fma(2.0, sm.B[pl.pu][(KH - 1) * TPL + h].y, qi[NI - 1]);
-                }
-                pair_term<NP, ODD, TPL, false>(qr, qi, -w, Pr, Pi, ar[KH - 1], ai[KH - 1]);            // (0, 1)
-#pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    x2r[p] += Pr[p];
-                    x2i[p] += Pi[p];
-                    const int a = 2 * p, c = 2 * p + 1;
-                    ar[a] = fma(Pr[p], sr[c], fma(-Pi[p], si[c], ar[a]));
-                    ai[a] = fma(Pr[p], si[c], fma(Pi[p], sr[c], ai[a]));
-                    ar[c] = fma(Pr[p], sr[a], fma(-Pi[p], si[a], ar[c]));
-                    ai[c] = fma(Pr[p], si[a], fma(Pi[p], sr[a], ai[c]));
-                }
+                pair_block<KH, TPL, double>(
+                    sr, si, Lur, Lui, Lvr, Lvi, w, ar, ai, x1r, x1i, x2r, x2i,
+                    [&](int p, double& re, double& im) {
+                        const double2 c = pt.C[2 * p * TPL + h];
+                        re = c.x;
+                        im = c.y;
+                    },
+                    [&](int d, double& re, double& im) {
+                        const double2 x = sm.B[d ? pl.pv : pl.pu][(KH - 1) * TPL + h];
+                        re = -2.0 * x.x;
+                        im = -2.0 * x.y;
+                    });
                 if (++i == Lin) break;
                 e = sm.tab_f[fwd ? i : Lin - i];           // backward: the transition into t + 1, undone
                 kd = (int)(e & 63u);

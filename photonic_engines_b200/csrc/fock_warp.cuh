@@ -67,18 +67,15 @@ static __device__ void prepare_warp(WS& sm, const double2* __restrict__ A, int m
             }
         }
     }
-    bool bin_in = true, bin_mid = true;             // schedules of radix-2 digits only (distinct rows)
-    for (int q = 0; q < pl.nin; ++q) bin_in = bin_in && pl.R[q] == 2;
-    for (int q = 0; q < pl.nmid; ++q) bin_mid = bin_mid && pl.R[pl.nin + q] == 2;
     for (int t = lane; t < pl.Lin; t += 32) {
         double w;
-        sm.tab_f[t] = gray_entry(pl, 0, pl.nin, pl.Pin, t, &w, t == pl.Lin - 1 ? sm.plan.vend : nullptr, bin_in);
+        sm.tab_f[t] = gray_entry(pl, 0, pl.nin, pl.Pin, t, &w, t == pl.Lin - 1 ? sm.plan.vend : nullptr, pl.ones_in);
         sm.tab_w[t] = w;
         sm.tab_w32[t] = (float)w;
     }
     for (int t = lane; t < pl.Lmid; t += 32) {
         double w;
-        sm.tab_fm[t] = gray_entry(pl, pl.nin, pl.nmid, pl.Pmid, t, &w, nullptr, bin_mid);
+        sm.tab_fm[t] = gray_entry(pl, pl.nin, pl.nmid, pl.Pmid, t, &w, nullptr, pl.ones_mid);
         sm.tab_wm[t] = w;
     }
 }
@@ -477,6 +474,17 @@ __device__ void chain_warp(const ChainParams& p, WS& sm, int64_t s) {
     __syncwarp();
     const double2* A = p.acol + off;
     const int kend = (p.k_stop > 0 && p.k_stop < nk) ? p.k_stop : nk;
+    double u_mine = 0.0;                                      // every step's uniform at once, one step per lane
+    if (lane >= kf - 1 && lane < kend) {
+        if (p.uniforms) {
+            u_mine = p.uniforms[s * p.n_stride + lane];
+        } else {
+            const int64_t row = p.seed_row ? p.seed_row[s] : 0;
+            const int64_t ro = p.rng_off ? p.rng_off[s] : s;
+            u_mine = chain_uniform((uint64_t)p.seeds[row * p.n_stride + lane], ro);
+        }
+    }
+    __syncwarp();
     for (int k = kf; k <= kend; ++k) {
         const int K1 = k - 1;
         if (K1 == 0) {
@@ -489,14 +497,7 @@ __device__ void chain_warp(const ChainParams& p, WS& sm, int64_t s) {
             __syncwarp();
             warp_cofactors<TPL, KPW, MIXED>(sm, k);
         }
-        double u;
-        if (p.uniforms) {
-            u = p.uniforms[s * p.n_stride + (k - 1)];
-        } else {
-            const int64_t row = p.seed_row ? p.seed_row[s] : 0;
-            const int64_t ro = p.rng_off ? p.rng_off[s] : s;
-            u = chain_uniform((uint64_t)p.seeds[row * p.n_stride + (k - 1)], ro);
-        }
+        const double u = __shfl_sync(0xffffffffu, u_mine, k - 1);
         double* mrow = p.marg ? p.marg + ((size_t)s * p.n_stride + (k - 1)) * p.marg_stride : nullptr;
         const double gap = draw_warp(sm, A, m, k, u, mrow);
         if constexpr (MIXED) {
@@ -505,8 +506,7 @@ __device__ void chain_warp(const ChainParams& p, WS& sm, int64_t s) {
                 draw_warp(sm, A, m, k, u, mrow);
             }
         }
-        if (lane == 0) add_to_groups(sm, sm.rows[k - 1]);
-        __syncwarp();
+        add_to_groups(sm, sm.rows[k - 1]);
     }
     for (int j = kf - 1 + lane; j < kend; j += 32) p.rows[s * p.n_stride + j] = sm.rows[j];
     if (p.occ && kend == nk) {

@@ -80,6 +80,7 @@ struct PlanT {
     int Pin[NK];      // prefix products of the inner radices
     int Pmid[NK];     // prefix products of the middle radices
     unsigned char vend[NK];   // inner digit values after a forward inner block
+    int ones_in, ones_mid;   // the schedules' digits all have radix 2 and multiplicity 1
     int pairs;        // two digits are taken out of the walk as u, v of the pair sweep (fock_pairs.cuh)
     int pu, pv;       // their kernel digits
     int sortR[NK];    // scratch of the planner: active digits by ascending radix
@@ -113,6 +114,7 @@ struct SmemT {
     double scan[MAX_WARPS];
     double fmin[MAX_WARPS];
     int cnt[MAX_WARPS];
+    double u[NK];                // the steps' uniforms
     int rows[NK];                // chosen modes so far
     int cols[NK];                // input columns of the stream in chain order
     int grow[NK];                // distinct chosen modes (groups), in order of first appearance
