@@ -192,9 +192,10 @@ __global__ void __launch_bounds__(1024) avoid_update_kernel(AvoidParams a) {
 }
 
 // Dynamic shared memory of a CTA: the tier's layout, then `weights` draw weights (0: a kernel without a draw); the
-// FP64 tiers up to 32 columns lay the pair sweep's tables over the weights.
+// FP64 and mixed tiers up to 32 columns lay the pair sweep's tables over the weights.
 static size_t cta_smem_bytes(int kpm, int prec, int weights) {
-    const size_t tables = (prec == PE_PRECISION_F64 && kpm <= NARROW) ? sizeof(PairTables<NARROW>) : 0;
+    const size_t tables = kpm > NARROW ? 0 : prec == PE_PRECISION_F64 ? sizeof(PairTables<NARROW>)
+                        : prec == PE_PRECISION_MIXED ? sizeof(PairTables32<NARROW>) : 0;
     const size_t w = (size_t)weights * sizeof(double);
     return smem_fixed_bytes_for(kpm, prec) + (w > tables ? w : tables);
 }

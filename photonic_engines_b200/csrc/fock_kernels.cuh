@@ -215,10 +215,11 @@ template <> struct TermCount<32> { typedef unsigned type; };
 // the middle block; what does not fit the schedules joins the lanes.  The ranking takes one ballot per
 // distinct radix value; the three splits are ballots over the ranks' prefix products (which only grow), and every
 // digit's table entries are written by the lane of its rank.
-// pair_lanes > 0: take two digits of multiplicity 1 out for the pair sweep of that many lanes, when there are
-// two; N then counts its blocks of four terms.
+// pair_lanes > 0: take two digits of multiplicity 1 out for the pair sweep of that many lanes (inner blocks of at
+// most pair_lin of its blocks), when there are two; N then counts its blocks of four terms.
 template <class SM>
-__device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid_max, int pair_lanes = 0) {
+__device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid_max, int pair_lanes = 0,
+                          int pair_lin = 0) {
     auto& pl = sm.plan;
     constexpr int GL = (SM::NKMAX + 31) / 32;          // groups (and ranks) per lane: index lane + 32 q, q < GL
     const unsigned full = 0xffffffffu;
@@ -242,7 +243,7 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
             if (ones && gu < 0) { gu = 32 * q + __ffs(ones) - 1; ones &= ones - 1u; }
             if (ones && gv < 0) gv = 32 * q + __ffs(ones) - 1;
         }
-        if (gv >= 0) lanes = pair_lanes;
+        if (gv >= 0) { lanes = pair_lanes; lin_max = pair_lin; }
         else gu = -1;                                  // fewer than two: the sweep term by term
     }
     int R[GL];
@@ -1054,9 +1055,10 @@ __device__ void sweep_mixed(SM& sm) {
     }
 
 // Steps of at least PAIRS_MIN columns run the pair sweep (fock_pairs.cuh) when their plan has its two digits, in
-// the kernels whose threads have 255 registers: lanes of two threads up to 20 columns, of four beyond, whatever
-// the term-by-term sweep's TPL.
+// the kernels whose threads have 255 registers: lanes of two threads up to 20 columns, of four beyond (mixed form:
+// half as many, each thread holding two such parts side by side), whatever the term-by-term sweep's TPL.
 constexpr int PAIRS_MIN = 9;
+constexpr int PAIRS_LIN32 = 128;       // mixed form: FP32 inner blocks of at most this many blocks of four terms
 template <int TPL, int KPM>
 __host__ __device__ constexpr bool has_pairs() {
     return PE_MAXT * PE_MINB <= 384 && TPL <= 2 && KPM >= PAIRS_MIN && KPM <= NARROW;
@@ -1103,9 +1105,13 @@ namespace pe {
 
 #define PE_PTIER(KPv)                                                                            \
     if constexpr (KPM >= KPv) {                                                                  \
-        if (K <= KPv) { sweep_pairs_f64<KPv / pair_tpl(KPv), pair_tpl(KPv)>(sm); return; }       \
+        if (K <= KPv) {                                                                          \
+            if constexpr (PREC == PREC_MIXED) sweep_pairs_mixed<KPv / pair_tpl(KPv), pair_tpl(KPv) / 2>(sm); \
+            else sweep_pairs_f64<KPv / pair_tpl(KPv), pair_tpl(KPv)>(sm);                        \
+            return;                                                                              \
+        }                                                                                        \
     }
-template <int KPM, class SM>
+template <int KPM, int PREC, class SM>
 __device__ void dispatch_pairs(SM& sm, int K) {
     PE_PTIER(12) PE_PTIER(16) PE_PTIER(20) PE_PTIER(24) PE_PTIER(28) PE_PTIER(32)
 }
@@ -1115,35 +1121,49 @@ __device__ void dispatch_pairs(SM& sm, int K) {
 template <int TPL, int KPM, int PREC, class SM>
 __device__ __forceinline__ void cofactor_step(SM& sm, const double2* A, int64_t rs, int64_t cs, int K1, int K) {
     constexpr bool MIXED = PREC == PREC_MIXED;
-    constexpr bool PAIRS = PREC == PREC_F64 && has_pairs<TPL, KPM>();
+    constexpr bool PAIRS = PREC != PREC_COMP && has_pairs<TPL, KPM>();
+    const int kp = (K + 3) / 4 * 4, ptl = pair_tpl(K) == 2 ? 1 : 2, pkh = kp >> ptl;
     if (threadIdx.x < 32)
         plan_step(sm, K1, K, blockDim.x / TPL * sm.lane_mult, MIXED ? MIXED_LIN : LIN_MAX, MID_MAX,
-                  PAIRS && K >= PAIRS_MIN ? blockDim.x / pair_tpl(K) * sm.lane_mult : 0);
+                  PAIRS && K >= PAIRS_MIN ? (blockDim.x >> (MIXED ? ptl - 1 : ptl)) * sm.lane_mult : 0,
+                  MIXED ? PAIRS_LIN32 : LIN_MAX);
     __syncthreads();
-    // paired FP32 sweeps (mixed form, 1- and 2-thread lanes): columns per thread of the dispatched tier
-    const int kh = (MIXED && PE_PAIR32 && TPL <= 2) ? ((K + 3) / 4 * 4) / TPL : 0;
     bool pairs = false;
     if constexpr (PAIRS) pairs = sm.plan.pairs;
-    const int ptl = pair_tpl(K) == 2 ? 1 : 2, pkh = ((K + 3) / 4 * 4) >> ptl;
-    prepare_step(sm, A, rs, cs, MIXED, kh, pairs ? pkh : 0, ptl);
+    // paired FP32 sweeps (mixed form, 1- and 2-thread lanes): columns per thread of the dispatched tier
+    const int kh = !MIXED ? 0 : pairs ? 2 * pkh : (PE_PAIR32 && TPL <= 2) ? kp / TPL : 0;
+    prepare_step(sm, A, rs, cs, MIXED, kh, pairs && !MIXED ? pkh : 0, ptl);
     __syncthreads();
     if constexpr (PREC == PREC_COMP) {
         prepare_comp(sm, ((K + 3) / 4 * 4) / TPL, TPL);
         __syncthreads();
         dispatch_comp<TPL, KPM>(sm, K);
-    } else if constexpr (MIXED) {
-        dispatch_mixed<TPL, KPM>(sm, K);
     } else {
         if constexpr (PAIRS) {
             if (pairs) {
-                prepare_pairs(sm, pkh, ptl);
+                if constexpr (MIXED) prepare_pairs32(sm, pkh, 1 << (ptl - 1));
+                else prepare_pairs(sm, pkh, ptl);
                 __syncthreads();
-                dispatch_pairs<KPM>(sm, K);
+                dispatch_pairs<KPM, PREC>(sm, K);
                 return;
             }
         }
-        dispatch_f64<TPL, KPM>(sm, K);
+        if constexpr (MIXED) dispatch_mixed<TPL, KPM>(sm, K);
+        else dispatch_f64<TPL, KPM>(sm, K);
     }
+}
+
+// The step again in FP64 (an FP32 form's draw inside the guard band), all threads.
+template <int TPL, int KPM, class SM>
+__device__ __forceinline__ void redo_step_f64(SM& sm, const double2* A, int64_t m, int K1, int K) {
+    if (sm.plan.pairs) {                               // the FP64 term-by-term sweep wants a plan of its own
+        __syncthreads();
+        if (threadIdx.x < 32) plan_step(sm, K1, K, blockDim.x / TPL * sm.lane_mult, LIN_MAX, MID_MAX);
+        __syncthreads();
+        prepare_step(sm, A, 1, m, false);
+        __syncthreads();
+    }
+    dispatch_f64<4, KPM>(sm, K);
 }
 
 // ---------------------------------------------------------------------------------------- draw
@@ -1306,7 +1326,7 @@ __device__ void chain_one(const ChainParams& p, SmemFor<KPM, PREC>& sm, double* 
         if constexpr (PREC != PREC_F64) {
             draw_step(sm, wgt, A, 1, m, m, k, u, mrow, false);
             if (K1 > 0 && sm.fmin[0] <= guard_band(p, k)) {   // uniform: read after the draw's final barrier
-                dispatch_f64<4, KPM>(sm, K);
+                redo_step_f64<TPL, KPM>(sm, A, m, K1, K);
                 draw_step(sm, wgt, A, 1, m, m, k, u, mrow, false);
             }
             if (tid < 32) add_to_groups(sm, sm.rows[k - 1]);

@@ -375,4 +375,186 @@ __device__ __forceinline__ void sweep_pairs_f64(SM& sm) {
     reduce_to_P<KH, TPL>(ar, ai, sm, c0);
 }
 
+// ---------------------------------------------------------------------------------------- mixed form
+// Step tables of the mixed form's pair walk, in the slots of B32: slot h KQ + r holds column h 2 KQ + r in .x / .z and
+// column h 2 KQ + KQ + r in .y / .w (real, imaginary).  Only the inner digits are walked in FP32.
+template <int NK>
+struct PairTables32 {
+    float4 G[NK][NK / 2];      // change of L_u (even r) and L_v (odd r) of the slot's pairs when the sums move by 2 B[kd]
+    float4 C[NK / 2];          // C of the pairs, at their even slot
+};
+template <class SM>
+__device__ __forceinline__ PairTables32<SM::NKMAX>& pair_tables32(const SM& sm) {
+    constexpr size_t at = (sizeof(SM) + 15) & ~(size_t)15;
+    return *reinterpret_cast<PairTables32<SM::NKMAX>*>(reinterpret_cast<unsigned char*>(const_cast<SM*>(&sm)) + at);
+}
+
+// x_a y_b + x_b y_a, complex: the mixed difference of the products of two columns.
+static __device__ __forceinline__ double2 cross(double2 xa, double2 xb, double2 ya, double2 yb) {
+    return make_double2(fma(xa.x, yb.x, -(xa.y * yb.y)) + fma(xb.x, ya.x, -(xb.y * ya.y)),
+                        fma(xa.x, yb.y, xa.y * yb.x) + fma(xb.x, ya.y, xb.y * ya.x));
+}
+
+// All threads, after B is complete (columns in order): kq columns per half thread, tpl threads per lane.
+template <class SM>
+static __device__ void prepare_pairs32(SM& sm, int kq, int tpl) {
+    const auto& pl = sm.plan;
+    auto& pt = pair_tables32(sm);
+    const int tid = threadIdx.x, T = blockDim.x, ns = kq * tpl;
+    const int nd = max(1, pl.nin);                         // row 0 is read (times zero) at a block's first term
+    for (int idx = tid; idx < nd * ns; idx += T) {
+        const int kd = idx / ns, q = idx % ns, r = q % kq;
+        if (r == kq - 1 && (kq & 1)) continue;
+        const int a = (q / kq) * 2 * kq + (r & ~1), d = (r & 1) ? pl.pv : pl.pu;
+        const double2 x = cross(sm.B[kd][a], sm.B[kd][a + 1], sm.B[d][a], sm.B[d][a + 1]);
+        const double2 y = cross(sm.B[kd][a + kq], sm.B[kd][a + kq + 1], sm.B[d][a + kq], sm.B[d][a + kq + 1]);
+        pt.G[kd][q] = make_float4((float)(-4.0 * x.x), (float)(-4.0 * y.x), (float)(-4.0 * x.y), (float)(-4.0 * y.y));
+    }
+    for (int q = tid; q < ns; q += T) {
+        const int r = q % kq;
+        if ((r & 1) || r == kq - 1) continue;
+        const int a = (q / kq) * 2 * kq + r;
+        const double2 x = cross(sm.B[pl.pu][a], sm.B[pl.pu][a + 1], sm.B[pl.pv][a], sm.B[pl.pv][a + 1]);
+        const double2 y = cross(sm.B[pl.pu][a + kq], sm.B[pl.pu][a + kq + 1], sm.B[pl.pv][a + kq], sm.B[pl.pv][a + kq + 1]);
+        pt.C[q] = make_float4((float)(4.0 * x.x), (float)(4.0 * y.x), (float)(4.0 * x.y), (float)(4.0 * y.y));
+    }
+}
+
+// The mixed form's pair sweep: as sweep_mixed, every inner block starts from column sums (and L_u, L_v) formed in
+// FP64 and rounded once, runs in complex FP32 on paired instructions (the thread's 2 KQ columns as two halves side by
+// side), and its shares of the cofactors, X_u and X_v are folded into FP64 accumulators.  A block walks a quarter of
+// the updates for the same terms, so its column sums drift less: largest marginal error against FP64 3.4e-5 -> 1.2e-5
+// at n = 20, m = 400 (256 chains), 9.3e-5 -> 4.5e-5 at n = 28, m = 784, largest CDF error halved.  n = 20, m = 400,
+// 2 000 streams 12.6 -> 9.9 ms; n = 24, m = 576, 600 streams 87 -> 70 ms; n = 28, m = 784, 148 streams 874 -> 768 ms.
+template <int KQ, int TPL, class SM>
+__device__ __forceinline__ void sweep_pairs_mixed(SM& sm) {
+    constexpr int NP = KQ / 2, KH = 2 * KQ;
+    const auto& pl = sm.plan;
+    const auto& pt = pair_tables32(sm);
+    const int tid = threadIdx.x;
+    const int lanes = blockDim.x / TPL, lane = tid / TPL, h = tid % TPL, c0 = h * KH;
+    const int wl0 = (tid & ~31) / TPL;
+    const int K = pl.K, Lin = pl.Lin, Lmid = pl.Lmid;
+    const int64_t H = pl.H;
+    double ar[KH], ai[KH];
+#pragma unroll
+    for (int j = 0; j < KH; ++j) { ar[j] = 0.0; ai[j] = 0.0; }
+    for (int64_t hw = sm.chunk * lanes + wl0; hw < H; hw += (int64_t)lanes * sm.lane_mult) {
+        double wh;
+        int64_t hl = hw + (lane - wl0);
+        const bool live = hl < H;
+        if (!live) hl = H - 1;
+        const uint64_t hpack = lane_digits(pl, hl, &wh);
+        if (!live) wh = 0.0;
+        for (int pm = 0; pm < Lmid; ++pm) {
+            const bool fwd = !(pm & 1);
+            float2 sr[KQ], si[KQ], Lur[NP], Lui[NP], Lvr[NP], Lvi[NP];
+            {
+                double xr[KH], xi[KH];
+                lane_sums<KH>(sm, c0, !fwd, pm, hl, hpack, xr, xi);
+#pragma unroll
+                for (int j = 0; j < KH; ++j) if (c0 + j >= K) { xr[j] = 1.0; xi[j] = 0.0; }
+#pragma unroll
+                for (int r = 0; r < KQ; ++r) {
+                    sr[r] = make_float2((float)xr[r], (float)xr[KQ + r]);
+                    si[r] = make_float2((float)xi[r], (float)xi[KQ + r]);
+                }
+                // L = -2 (s_a d_b + s_b d_a) + 4 d_a d_b = -2 ((s_b - d_b) d_a + (s_a - d_a) d_b) for the row d of u
+                // or v, and C = 4 (u_a v_b + u_b v_a) added to L_v
+                auto lin = [&](int d, int a, bool withc) {
+                    const double2 da = sm.B[d][c0 + a], db = sm.B[d][c0 + a + 1];
+                    const double2 x = cross(make_double2(xr[a] - da.x, xi[a] - da.y),
+                                            make_double2(xr[a + 1] - db.x, xi[a + 1] - db.y), da, db);
+                    double2 l = make_double2(-2.0 * x.x, -2.0 * x.y);
+                    if (withc) {
+                        const double2 c = cross(sm.B[pl.pu][c0 + a], sm.B[pl.pu][c0 + a + 1], da, db);
+                        l = make_double2(fma(4.0, c.x, l.x), fma(4.0, c.y, l.y));
+                    }
+                    return l;
+                };
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    const double2 ux = lin(pl.pu, 2 * p, false), uy = lin(pl.pu, KQ + 2 * p, false);
+                    const double2 vx = lin(pl.pv, 2 * p, true), vy = lin(pl.pv, KQ + 2 * p, true);
+                    Lur[p] = make_float2((float)ux.x, (float)uy.x);
+                    Lui[p] = make_float2((float)ux.y, (float)uy.y);
+                    Lvr[p] = make_float2((float)vx.x, (float)vy.x);
+                    Lvi[p] = make_float2((float)vx.y, (float)vy.y);
+                }
+            }
+            float2 a2r[KQ], a2i[KQ], x1r[NP], x1i[NP], x2r[NP], x2i[NP];
+#pragma unroll
+            for (int r = 0; r < KQ; ++r) { a2r[r] = make_float2(0.0f, 0.0f); a2i[r] = make_float2(0.0f, 0.0f); }
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                x1r[p] = make_float2(0.0f, 0.0f); x1i[p] = make_float2(0.0f, 0.0f);
+                x2r[p] = make_float2(0.0f, 0.0f); x2i[p] = make_float2(0.0f, 0.0f);
+            }
+            unsigned e = 0u;
+            float f = 0.0f;                                // no transition into the block's first term
+            int kd = 0;
+            for (int i = 0;;) {
+                const int t = fwd ? i : Lin - 1 - i;
+                const float4* b = reinterpret_cast<const float4*>(&sm.B32[kd][0]) + h * KQ;
+                const float4* g = &pt.G[kd][h * KQ];
+                const float2 ff = make_float2(f, f);
+#pragma unroll
+                for (int r = 0; r < KQ; ++r) {
+                    const float4 v = b[r];
+                    sr[r] = vfma(ff, make_float2(v.x, v.y), sr[r]);
+                    si[r] = vfma(ff, make_float2(v.z, v.w), si[r]);
+                }
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    const float4 u = g[2 * p], v = g[2 * p + 1];
+                    Lur[p] = vfma(ff, make_float2(u.x, u.y), Lur[p]);
+                    Lui[p] = vfma(ff, make_float2(u.z, u.w), Lui[p]);
+                    Lvr[p] = vfma(ff, make_float2(v.x, v.y), Lvr[p]);
+                    Lvi[p] = vfma(ff, make_float2(v.z, v.w), Lvi[p]);
+                }
+                const float w = sm.tab_w32[t];
+                pair_block<KQ, TPL, float2>(
+                    sr, si, Lur, Lui, Lvr, Lvi, make_float2(w, w), a2r, a2i, x1r, x1i, x2r, x2i,
+                    [&](int p, float2& re, float2& im) {
+                        const float4 c = pt.C[h * KQ + 2 * p];
+                        re = make_float2(c.x, c.y);
+                        im = make_float2(c.z, c.w);
+                    },
+                    [&](int d, float2& re, float2& im) {
+                        const float4 x = reinterpret_cast<const float4*>(&sm.B32[d ? pl.pv : pl.pu][0])[h * KQ + KQ - 1];
+                        re = make_float2(-x.x, -x.y);
+                        im = make_float2(-x.z, -x.w);
+                    });
+                if (++i == Lin) break;
+                e = sm.tab_f[fwd ? i : Lin - i];
+                kd = (int)(e & 63u);
+                f = (((e & 0x80u) != 0u) == fwd) ? -1.0f : 1.0f;
+            }
+            const double wmh = wh * sm.tab_wm[pm];
+#pragma unroll
+            for (int r = 0; r < KQ; ++r) {
+                ar[r] = fma(wmh, (double)a2r[r].x, ar[r]);
+                ai[r] = fma(wmh, (double)a2i[r].x, ai[r]);
+                ar[KQ + r] = fma(wmh, (double)a2r[r].y, ar[KQ + r]);
+                ai[KQ + r] = fma(wmh, (double)a2i[r].y, ai[KQ + r]);
+            }
+#pragma unroll
+            for (int r = 0; r < 2 * NP; ++r) {
+                const int p = r / 2;
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    const double2 u = sm.B[pl.pu][c0 + y * KQ + (r ^ 1)], v = sm.B[pl.pv][c0 + y * KQ + (r ^ 1)];
+                    const double Xr = y ? x1r[p].y : x1r[p].x, Xi = y ? x1i[p].y : x1i[p].x;
+                    const double Yr = y ? x2r[p].y : x2r[p].x, Yi = y ? x2i[p].y : x2i[p].x;
+                    const double tr = fma(u.x, Xr, fma(-u.y, Xi, fma(v.x, Yr, -(v.y * Yi))));
+                    const double ti = fma(u.x, Xi, fma(u.y, Xr, fma(v.x, Yi, v.y * Yr)));
+                    ar[y * KQ + r] = fma(-2.0 * wmh, tr, ar[y * KQ + r]);
+                    ai[y * KQ + r] = fma(-2.0 * wmh, ti, ai[y * KQ + r]);
+                }
+            }
+        }
+    }
+    reduce_to_P<KH, TPL>(ar, ai, sm, c0);
+}
+
 }  // namespace pe
