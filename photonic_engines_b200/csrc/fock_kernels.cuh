@@ -1100,14 +1100,15 @@ __device__ void dispatch_mixed(SM& sm, int K) {
 
 #include "fock_comp.cuh"
 #include "fock_pairs.cuh"
+#include "fock_direct.cuh"
 
 namespace pe {
 
 #define PE_PTIER(KPv)                                                                            \
     if constexpr (KPM >= KPv) {                                                                  \
         if (K <= KPv) {                                                                          \
-            if constexpr (PREC == PREC_MIXED) sweep_pairs_mixed<KPv / pair_tpl(KPv), pair_tpl(KPv) / 2>(sm); \
-            else sweep_pairs_f64<KPv / pair_tpl(KPv), pair_tpl(KPv)>(sm);                        \
+            if constexpr (PREC == PREC_MIXED) sweep_pairs_mixed<KPv / pair_tpl(KPv), pair_tpl(KPv) / 2, SM>(); \
+            else sweep_pairs_f64<KPv / pair_tpl(KPv), pair_tpl(KPv), SM>();                        \
             return;                                                                              \
         }                                                                                        \
     }
@@ -1169,12 +1170,14 @@ __device__ __forceinline__ void redo_step_f64(SM& sm, const double2* A, int64_t 
 // ---------------------------------------------------------------------------------------- draw
 // Marginal over the m output modes, FP64 block scan (contiguous chunk per thread, warp scan, warps
 // in order), then idx = min(#{rho : cw_rho < u * tot}, m - 1) with tot = cw[m - 1]
-// (cofactors_triton.py:298-308).  Warp 0 records the pick and updates the groups; the gap
-// min |cw - u tot| / tot is left in sm.fmin[0].
-template <class SM>
-static __device__ void draw_step(SM& sm, double* __restrict__ wgt, const double2* __restrict__ A, int64_t rs, int64_t cs,
-                                 int m, int k, double u, double* __restrict__ marg_row, bool update_groups) {
+// (cofactors_triton.py:298-308).  All threads return the pick, and (GAP) the gap min |cw - u tot| / tot; thread 0 has
+// written it to sm.rows and warp 0 (groups) added it to the groups, with no barrier after that.  Three barriers: short
+// steps are bound by them and by the latencies between them.
+template <bool GAP, class SM>
+static __device__ int draw_step(SM& sm, double* __restrict__ wgt, const double2* __restrict__ A, int64_t rs, int64_t cs,
+                                int m, int k, double u, double* __restrict__ marg_row, bool groups, double* gap) {
     const int tid = threadIdx.x, T = blockDim.x, lid = tid & 31, wid = tid >> 5, nw = T >> 5;
+    if (tid == 0) { sm.below = 0; sm.gap_bits = 0x7fefffffffffffffll; }
     // DR modes per thread at a time, and the column loop unrolled DC times, so that 16 or 32 independent loads of
     // A (from L2) are in flight instead of one; the sum over columns keeps its order (same bits as one mode
     // at a time).  The draw is bound by L2 latency, not by its few FLOPs (m = 900, the c3 batch: 4-5 %
@@ -1223,17 +1226,14 @@ static __device__ void draw_step(SM& sm, double* __restrict__ wgt, const double2
     if (lid == 0) excl = 0.0;
     if (lid == 31) sm.scan[wid] = x;
     __syncthreads();
-    double E = 0.0;
-    for (int w = 0; w < wid; ++w) E += sm.scan[w];
-    E += excl;
-    if (lo <= m - 1 && m - 1 < hi) {
-        double cw = E;
-        for (int i = lo; i < hi; ++i) cw += wgt[i];
-        sm.tot = cw;
-        sm.target = u * cw;
+    double E = 0.0, tot = 0.0;
+#pragma unroll
+    for (int w = 0; w < MAX_WARPS; ++w) {
+        if (w == wid) E = tot;
+        if (w < nw) tot += sm.scan[w];
     }
-    __syncthreads();
-    const double tot = sm.tot, target = sm.target;
+    E += excl;
+    const double target = u * tot;
     int cnt = 0;
     double gmin = 1.0e300;
     {
@@ -1241,31 +1241,23 @@ static __device__ void draw_step(SM& sm, double* __restrict__ wgt, const double2
         for (int i = lo; i < hi; ++i) {
             cw += wgt[i];
             cnt += (cw < target) ? 1 : 0;
-            gmin = fmin(gmin, fabs(cw - target));
+            if (GAP) gmin = fmin(gmin, fabs(cw - target));
         }
     }
     if (marg_row) for (int rho = tid; rho < m; rho += T) marg_row[rho] = wgt[rho] / tot;
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lid == 0 && cnt > 0) atomicAdd(&sm.below, cnt);
+    if (GAP) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        gmin = fmin(gmin, __shfl_xor_sync(0xffffffffu, gmin, o));
-    }
-    if (lid == 0) { sm.cnt[wid] = cnt; sm.fmin[wid] = gmin; }
-    __syncthreads();
-    if (wid == 0) {
-        int c = lid < nw ? sm.cnt[lid] : 0;
-        double g = lid < nw ? sm.fmin[lid] : 1.0e300;
-        c = __reduce_add_sync(0xffffffffu, c);
-#pragma unroll
-        for (int o = MAX_WARPS / 2; o > 0; o >>= 1) g = fmin(g, __shfl_xor_sync(0xffffffffu, g, o));
-        const int pick = min(c, m - 1);
-        if (lid == 0) {
-            sm.rows[k - 1] = pick;
-            sm.fmin[0] = g / tot;
-        }
-        if (update_groups) add_to_groups(sm, pick);
+        for (int o = 16; o > 0; o >>= 1) gmin = fmin(gmin, __shfl_xor_sync(0xffffffffu, gmin, o));
+        if (lid == 0) atomicMin(&sm.gap_bits, __double_as_longlong(gmin));       // non-negative: ordered as integers
     }
     __syncthreads();
+    const int pick = min(sm.below, m - 1);
+    if (GAP) *gap = __longlong_as_double(sm.gap_bits) / tot;
+    if (tid == 0) sm.rows[k - 1] = pick;
+    if (groups && wid == 0) add_to_groups(sm, pick);
+    return pick;
 }
 
 // ---------------------------------------------------------------------------------------- chain
@@ -1307,34 +1299,46 @@ __device__ void chain_one(const ChainParams& p, SmemFor<KPM, PREC>& sm, double* 
         if (tid == 0) record_error(p.status, p.detail, s);
         return;
     }
-    if (kf > 1) {
-        if (tid < 32) build_groups_warp(sm, kf - 1);
-        __syncthreads();
-    }
     const double2* A = p.acol + off;      // (rho, j) at A[j * m + rho]
+    if (kf > 1 && tid < 32) {             // warp 0 alone: groups and direct rows are its own
+        if (kf > DIRECT_MAX) build_groups_warp(sm, kf - 1);
+        else load_rows(sm, A, 1, m, 0, kf - 1, nk);
+        __syncwarp();
+    }
     const int kend = (stop_early && p.k_stop > 0 && p.k_stop < nk) ? p.k_stop : nk;
     for (int k = kf; k <= kend; ++k) {
         const int K = k, K1 = k - 1;
         if (K1 == 0) {
             if (tid == 0) sm.P[0] = make_double2(1.0, 0.0);
             __syncthreads();
+        } else if (K <= DIRECT_MAX) {
+            if (tid < 32) cofactors_direct(sm, K);
+            __syncthreads();
         } else {
             cofactor_step<TPL, KPM, PREC>(sm, A, 1, m, K1, K);
         }
         const double u = sm.u[k - 1];
         double* mrow = p.marg ? p.marg + ((size_t)s * p.n_stride + (k - 1)) * p.marg_stride : nullptr;
+        const bool planned = k > DIRECT_MAX;            // this step kept the groups; the first planned step builds them
         if constexpr (PREC != PREC_F64) {
-            draw_step(sm, wgt, A, 1, m, m, k, u, mrow, false);
-            if (K1 > 0 && sm.fmin[0] <= guard_band(p, k)) {   // uniform: read after the draw's final barrier
+            double gap;
+            int pick = draw_step<true>(sm, wgt, A, 1, m, m, k, u, mrow, false, &gap);
+            if (planned && gap <= guard_band(p, k)) {   // uniform
                 redo_step_f64<TPL, KPM>(sm, A, m, K1, K);
-                draw_step(sm, wgt, A, 1, m, m, k, u, mrow, false);
+                pick = draw_step<true>(sm, wgt, A, 1, m, m, k, u, mrow, false, &gap);
             }
-            if (tid < 32) add_to_groups(sm, sm.rows[k - 1]);
-            __syncthreads();
+            if (planned && tid < 32) add_to_groups(sm, pick);
         } else {
-            draw_step(sm, wgt, A, 1, m, m, k, u, mrow, true);
+            draw_step<false>(sm, wgt, A, 1, m, m, k, u, mrow, planned, nullptr);
+        }
+        if (!planned && k < kend && tid < 32) {
+            __syncwarp();                               // thread 0 has written the pick
+            if (k == DIRECT_MAX) build_groups_warp(sm, k);
+            else load_rows(sm, A, 1, m, k - 1, k, nk);
+            __syncwarp();
         }
     }
+    __syncthreads();
     for (int j = kf - 1 + tid; j < kend; j += blockDim.x) p.rows[s * p.n_stride + j] = sm.rows[j];
     if (p.occ && kend == nk) {
         for (int rho = tid; rho < p.occ_stride; rho += blockDim.x) {
@@ -1498,14 +1502,17 @@ __global__ void __launch_bounds__(PE_MAXT, PE_MINB) split_draw_kernel(SplitParam
             u = chain_uniform((uint64_t)p.seeds[row * p.n_stride + (k - 1)], ro);
         }
         double* mrow = p.marg ? p.marg + ((size_t)s * p.n_stride + (k - 1)) * p.marg_stride : nullptr;
-        draw_step(sm, wgt, A, 1, m, m, k, u, mrow, false);
         if constexpr (PREC != PREC_F64) {
-            const bool redo = sm.fmin[0] <= guard_band(p, k);   // guard band: the FP64 pass redoes this step
+            double gap;
+            draw_step<true>(sm, wgt, A, 1, m, m, k, u, mrow, false, &gap);
+            const bool redo = gap <= guard_band(p, k);          // guard band: the FP64 pass redoes this step
             if (tid == 0) sp.flag[q] = redo ? 1 : 0;
             if (redo) { __syncthreads(); continue; }
         } else {
+            draw_step<false>(sm, wgt, A, 1, m, m, k, u, mrow, false, nullptr);
             if (sp.pass == 1 && tid == 0) sp.flag[q] = 0;
         }
+        __syncthreads();                                        // the pick, for the occupations
         if (tid == 0) p.rows[s * p.n_stride + (k - 1)] = sm.rows[k - 1];
         const int nk = p.nk ? p.nk[s] : p.n_stride;
         if (p.occ && k == nk) {
@@ -1528,6 +1535,31 @@ __global__ void __launch_bounds__(256) cofactor_kernel(const double2* __restrict
     using SM = SmemFor<KPM, PREC>;
     SM& sm = *reinterpret_cast<SM*>(smem_raw);
     const int tid = threadIdx.x;
+    if (K > 1 && K <= DIRECT_MAX) {                             // one warp per block, no plan
+        static_assert(MAX_WARPS * sizeof(DirectSmem) <= sizeof(SM), "a slice per warp");
+        const int nw = blockDim.x >> 5, lane = tid & 31;
+        DirectSmem& ws = reinterpret_cast<DirectSmem*>(smem_raw)[tid >> 5];
+        for (int64_t s = (int64_t)blockIdx.x * nw + (tid >> 5); s < S; s += (int64_t)gridDim.x * nw) {
+            bool bad = false;
+            if (lane < K - 1) {
+                const int64_t r = rows[s * (K - 1) + lane];
+                bad = r < 0 || r >= m;
+                ws.rows[lane] = (int)r;
+            }
+            if (lane < K) ws.cols[lane] = lane;
+            if (__any_sync(0xffffffffu, bad)) {
+                if (lane == 0) record_error(status, detail, s);
+                continue;
+            }
+            __syncwarp();
+            load_rows(ws, A + s * (int64_t)m * K, K, 1, 0, K - 1, K);
+            __syncwarp();
+            cofactors_direct(ws, K);
+            if (lane < K) P[s * K + lane] = ws.P[lane];
+            __syncwarp();
+        }
+        return;
+    }
     for (int64_t s = blockIdx.x; s < S; s += gridDim.x) {
         if (tid == 0) { sm.bad = 0; sm.ngrp = 0; sm.chunk = 0; sm.lane_mult = 1; }
         __syncthreads();

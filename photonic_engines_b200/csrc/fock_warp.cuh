@@ -14,9 +14,8 @@ constexpr int WMAXN = 16;      // photons per stream
 constexpr int WLIN = 128;      // inner schedule length
 constexpr int WMID = 128;      // middle schedule length
 constexpr int WARPS = 8;       // warps (streams in flight) per CTA
-constexpr int WDIRECT = 8;     // steps of at most this many columns sum over the chosen rows themselves
 
-// A stream's slice of shared memory: what every step needs, and for kernels beyond WDIRECT columns the plan and
+// A stream's slice of shared memory: what every step needs, and for kernels beyond DIRECT_MAX columns the plan and
 // schedules of the collapsed sum.
 template <int NK>
 struct WarpSmemBase {
@@ -27,7 +26,7 @@ struct WarpSmemBase {
     int cols[NK];
     int64_t cur;
 };
-template <int NK, bool DIRECT = (NK <= WDIRECT)>
+template <int NK, bool DIRECT = (NK <= DIRECT_MAX)>
 struct WarpSmemT : WarpSmemBase<NK> {};
 template <int NK>
 struct WarpSmemT<NK, false> : WarpSmemBase<NK> {
@@ -43,94 +42,6 @@ struct WarpSmemT<NK, false> : WarpSmemBase<NK> {
     int ngrp;
 };
 using WarpSmem = WarpSmemT<WMAXN>;    // the largest slice (streams of up to 16 photons)
-
-// ---------------------------------------------------------------------------------------- direct steps
-// Row k - 1 (the mode just chosen) of the stream's instance into row k - 1 of B, every input column of the chain at
-// once: the direct steps after it read their block from shared memory.
-template <class WS>
-static __device__ __forceinline__ void load_row(WS& sm, const double2* __restrict__ A, int m, int i, int row, int nk) {
-    const int lane = threadIdx.x & 31;
-    if (lane < nk) sm.B[i][lane] = A[(int64_t)row + (int64_t)sm.cols[lane] * m];
-}
-
-// Cofactors of a step of K <= 2 KH columns, FP64: Glynn's sum over the 2^(K1 - 1) sign vectors of the K1 chosen
-// rows as they are (repeated rows are not collapsed: at most 64 terms, a few per lane), two threads per sign vector
-// and 16 sign vectors at a time.  No multiplicities, plan or schedules: chains this short are bound by the
-// instructions of that set-up, not by the sum (FP64 pipe 11 % busy with it; n = 6, m = 12: about 1 200 warp
-// instructions per step with the collapsed sum, a third of it here).  The sum over the lanes is halved: every
-// exchange carries half of the values still held.
-template <int KH, class WS>
-__device__ __forceinline__ void cofactors_direct(WS& sm, int K) {
-    const int lid = threadIdx.x & 31, h = lid & 1, c0 = h * KH, K1 = K - 1;
-    const int N = 1 << (K1 - 1);
-    double ar[KH], ai[KH];
-#pragma unroll
-    for (int j = 0; j < KH; ++j) { ar[j] = 0.0; ai[j] = 0.0; }
-    for (int t0 = 0; t0 < N; t0 += 16) {
-        const int t = t0 + (lid >> 1);
-        double sr[KH], si[KH];
-#pragma unroll
-        for (int j = 0; j < KH; ++j) {
-            const double2 b = sm.B[0][c0 + j];
-            sr[j] = b.x;
-            si[j] = b.y;
-        }
-        for (int i = 1; i < K1; ++i) {
-            const double d = ((t >> (i - 1)) & 1) ? -1.0 : 1.0;
-#pragma unroll
-            for (int j = 0; j < KH; ++j) {
-                const double2 b = sm.B[i][c0 + j];
-                sr[j] = fma(d, b.x, sr[j]);
-                si[j] = fma(d, b.y, si[j]);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < KH; ++j)                       // columns past K count as 1 (their B may be unset)
-            if (c0 + j >= K) { sr[j] = 1.0; si[j] = 0.0; }
-        const double w = t >= N ? 0.0 : ((__popc(t) & 1) ? -1.0 : 1.0);
-        term<KH, 2, double, double2>(sr, si, ar, ai, nullptr, 0.0, w, h, 0xffffffffu);
-    }
-    // lanes with bit 4 clear keep the real parts, the others the imaginary ones; then (KH 2, 4) half of the columns
-    const bool im = (lid & 16) != 0;
-    double v[KH];
-#pragma unroll
-    for (int j = 0; j < KH; ++j) {
-        const double give = im ? ar[j] : ai[j];
-        v[j] = (im ? ai[j] : ar[j]) + __shfl_xor_sync(0xffffffffu, give, 16);
-    }
-    const double scale = __longlong_as_double((long long)(1023 - (K1 - 1)) << 52);      // 2^-(K1 - 1)
-    double* P = reinterpret_cast<double*>(&sm.P[0]);
-    if constexpr (KH % 2 == 0) {
-        constexpr int KQ = KH / 2;
-        const int up = (lid >> 3) & 1;
-        double x[KQ];
-#pragma unroll
-        for (int j = 0; j < KQ; ++j) {
-            const double give = up ? v[j] : v[KQ + j];
-            x[j] = (up ? v[KQ + j] : v[j]) + __shfl_xor_sync(0xffffffffu, give, 8);
-        }
-        double y;
-        int col = c0 + up * KQ;
-        if constexpr (KQ == 2) {
-            const int up2 = (lid >> 2) & 1;
-            const double give = up2 ? x[0] : x[1];
-            y = (up2 ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, give, 4);
-            col += up2;
-        } else {
-            y = x[0] + __shfl_xor_sync(0xffffffffu, x[0], 4);
-        }
-        y += __shfl_xor_sync(0xffffffffu, y, 2);
-        if (!(lid & 2) && (KQ == 2 || !(lid & 4))) P[2 * col + (im ? 1 : 0)] = y * scale;
-    } else {
-#pragma unroll
-        for (int j = 0; j < KH; ++j) {
-#pragma unroll
-            for (int o = 8; o > 1; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-            if (!(lid & 14)) P[2 * (c0 + j) + (im ? 1 : 0)] = v[j] * scale;
-        }
-    }
-    __syncwarp();
-}
 
 // Gather B and fill the schedules, lane-parallel.  Element (rho, j) of the instance is A[rho + j * m].
 template <class WS>
@@ -283,7 +194,7 @@ __device__ void sweep_warp_mixed(WS& sm) {
         if (K <= KPv) { CALL; return; }                      \
     }
 
-// A planned step (more than WDIRECT columns).
+// A planned step (more than DIRECT_MAX columns).
 template <int TPL, int KPW, bool MIXED, class WS>
 __device__ void warp_cofactors(WS& sm, int K) {
     if constexpr (MIXED) {
@@ -574,19 +485,17 @@ __device__ void chain_warp(const ChainParams& p, WS& sm, int64_t s) {
             u_mine = chain_uniform((uint64_t)p.seeds[row * p.n_stride + lane], ro);
         }
     }
-    for (int i = 0; i < kf - 1 && i < WDIRECT - 1; ++i) load_row(sm, A, m, i, sm.rows[i], nk);
+    load_rows(sm, A, 1, m, 0, min(kf - 1, DIRECT_MAX - 1), nk);
     __syncwarp();
     for (int k = kf; k <= kend; ++k) {
         const int K1 = k - 1;
-        const bool direct = k <= WDIRECT;
+        const bool direct = k <= DIRECT_MAX;
         if (K1 == 0) {
             if (lane == 0) sm.P[0] = make_double2(1.0, 0.0);
             __syncwarp();
         } else if (direct) {
-            if (k <= 4) cofactors_direct<2>(sm, k);
-            else if (k <= 6) cofactors_direct<3>(sm, k);
-            else cofactors_direct<4>(sm, k);
-        } else if constexpr (KPW > WDIRECT) {
+            cofactors_direct(sm, k);
+        } else if constexpr (KPW > DIRECT_MAX) {
             build_groups_warp(sm, K1);
             __syncwarp();
             plan_step(sm, K1, k, 32 / TPL, WLIN, WMID);
@@ -598,13 +507,13 @@ __device__ void chain_warp(const ChainParams& p, WS& sm, int64_t s) {
         const double u = __shfl_sync(0xffffffffu, u_mine, k - 1);
         double* mrow = p.marg ? p.marg + ((size_t)s * p.n_stride + (k - 1)) * p.marg_stride : nullptr;
         const double gap = draw_warp(sm, A, m, k, u, mrow);
-        if constexpr (MIXED && KPW > WDIRECT) {
+        if constexpr (MIXED && KPW > DIRECT_MAX) {
             if (!direct && gap <= guard_band(p, k)) {       // guard band: this step again in FP64
                 warp_cofactors<TPL, KPW, false>(sm, k);
                 draw_warp(sm, A, m, k, u, mrow);
             }
         }
-        if (k < kend && k < WDIRECT) load_row(sm, A, m, k - 1, sm.rows[k - 1], nk);
+        if (k < kend && k < DIRECT_MAX) load_rows(sm, A, 1, m, k - 1, k, nk);
         __syncwarp();
     }
     for (int j = kf - 1 + lane; j < kend; j += 32) p.rows[s * p.n_stride + j] = sm.rows[j];

@@ -112,8 +112,8 @@ struct SmemT {
     unsigned char tab_fm[MID_MAX]; // transition into middle index: middle digit | 0x80 when -2 b
     double2 red[MAX_WARPS][NK];  // cross-warp reduction
     double scan[MAX_WARPS];
-    double fmin[MAX_WARPS];
-    int cnt[MAX_WARPS];
+    long long gap_bits;          // the draw: smallest distance of the cumulative weights to u tot (bits of a double)
+    int below;                   // and how many of them lie below it
     double u[NK];                // the steps' uniforms
     int rows[NK];                // chosen modes so far
     int cols[NK];                // input columns of the stream in chain order
@@ -123,7 +123,6 @@ struct SmemT {
     int64_t cur;                   // stream being processed (-1: queue drained)
     int64_t chunk;                 // this CTA's chunk of the Gray lanes (split steps; 0 else)
     int lane_mult;                 // CTAs sharing one step of a stream (1 unless the step is split)
-    double tot, target;
     int bad;                       // set by any thread that saw an out-of-range index
 };
 
