@@ -216,10 +216,10 @@ template <> struct TermCount<32> { typedef unsigned type; };
 // distinct radix value; the three splits are ballots over the ranks' prefix products (which only grow), and every
 // digit's table entries are written by the lane of its rank.
 // pair_lanes > 0: take two digits of multiplicity 1 out for the pair sweep of that many lanes (inner blocks of at
-// most pair_lin of its blocks), when there are two; N then counts its blocks of four terms.
+// most pair_lin of its blocks), when there are pair_min >= 2; N then counts its blocks of four terms.
 template <class SM>
 __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid_max, int pair_lanes = 0,
-                          int pair_lin = 0) {
+                          int pair_lin = 0, int pair_min = 2) {
     auto& pl = sm.plan;
     constexpr int GL = (SM::NKMAX + 31) / 32;          // groups (and ranks) per lane: index lane + 32 q, q < GL
     const unsigned full = 0xffffffffu;
@@ -234,17 +234,18 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
         if (oddmask) halved = 32 * q + 31 - __clz(oddmask);
     }
     // the pair sweep's digits u, v: the first two groups of multiplicity 1 (the halved one aside)
-    int gu = -1, gv = -1;
+    int gu = -1, gv = -1, nones = 0;
     if (pair_lanes > 0) {
 #pragma unroll
         for (int q = 0; q < GL; ++q) {
             const int g = lane + 32 * q;
             unsigned ones = __ballot_sync(full, g < D && g != halved && sm.gmul[g < D ? g : 0] == 1);
+            nones += __popc(ones);
             if (ones && gu < 0) { gu = 32 * q + __ffs(ones) - 1; ones &= ones - 1u; }
             if (ones && gv < 0) gv = 32 * q + __ffs(ones) - 1;
         }
-        if (gv >= 0) { lanes = pair_lanes; lin_max = pair_lin; }
-        else gu = -1;                                  // fewer than two: the sweep term by term
+        if (nones >= pair_min) { lanes = pair_lanes; lin_max = pair_lin; }
+        else { gu = -1; gv = -1; }                     // too few: the sweep term by term
     }
     int R[GL];
     bool active[GL];
@@ -1059,6 +1060,10 @@ __device__ void sweep_mixed(SM& sm) {
 // half as many, each thread holding two such parts side by side), whatever the term-by-term sweep's TPL.
 constexpr int PAIRS_MIN = 9;
 constexpr int PAIRS_LIN32 = 128;       // mixed form: FP32 inner blocks of at most this many blocks of four terms
+// Mixed form: modes chosen once that a step needs for the pair sweep.  A more crowded step's terms cancel to 1e-3 of
+// their size and less; there the FP32 blocks' error is a matter of luck in either sweep (27 rows on 10 modes: at most
+// 3e-3 of the cofactors in both, 7e-5 in the median), there are few terms, and the older sweep stays.
+constexpr int PAIRS_ONES32 = 6;
 template <int TPL, int KPM>
 __host__ __device__ constexpr bool has_pairs() {
     return PE_MAXT * PE_MINB <= 384 && TPL <= 2 && KPM >= PAIRS_MIN && KPM <= NARROW;
@@ -1127,7 +1132,7 @@ __device__ __forceinline__ void cofactor_step(SM& sm, const double2* A, int64_t 
     if (threadIdx.x < 32)
         plan_step(sm, K1, K, blockDim.x / TPL * sm.lane_mult, MIXED ? MIXED_LIN : LIN_MAX, MID_MAX,
                   PAIRS && K >= PAIRS_MIN ? (blockDim.x >> (MIXED ? ptl - 1 : ptl)) * sm.lane_mult : 0,
-                  MIXED ? PAIRS_LIN32 : LIN_MAX);
+                  MIXED ? PAIRS_LIN32 : LIN_MAX, MIXED ? PAIRS_ONES32 : 2);
     __syncthreads();
     bool pairs = false;
     if constexpr (PAIRS) pairs = sm.plan.pairs;
