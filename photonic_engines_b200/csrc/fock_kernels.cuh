@@ -1307,7 +1307,7 @@ __device__ void chain_one(const ChainParams& p, SmemFor<KPM, PREC>& sm, double* 
     const double2* A = p.acol + off;      // (rho, j) at A[j * m + rho]
     if (kf > 1 && tid < 32) {             // warp 0 alone: groups and direct rows are its own
         if (kf > DIRECT_MAX) build_groups_warp(sm, kf - 1);
-        else load_rows(sm, A, 1, m, 0, kf - 1, nk);
+        else load_rows<DIRECT_MAX>(sm, A, 1, m, 0, kf - 1, nk);
         __syncwarp();
     }
     const int kend = (stop_early && p.k_stop > 0 && p.k_stop < nk) ? p.k_stop : nk;
@@ -1317,7 +1317,7 @@ __device__ void chain_one(const ChainParams& p, SmemFor<KPM, PREC>& sm, double* 
             if (tid == 0) sm.P[0] = make_double2(1.0, 0.0);
             __syncthreads();
         } else if (K <= DIRECT_MAX) {
-            if (tid < 32) cofactors_direct(sm, K);
+            if (tid < 32) cofactors_direct<DIRECT_MAX>(sm, K);
             __syncthreads();
         } else {
             cofactor_step<TPL, KPM, PREC>(sm, A, 1, m, K1, K);
@@ -1339,7 +1339,7 @@ __device__ void chain_one(const ChainParams& p, SmemFor<KPM, PREC>& sm, double* 
         if (!planned && k < kend && tid < 32) {
             __syncwarp();                               // thread 0 has written the pick
             if (k == DIRECT_MAX) build_groups_warp(sm, k);
-            else load_rows(sm, A, 1, m, k - 1, k, nk);
+            else load_rows<DIRECT_MAX>(sm, A, 1, m, k - 1, k, nk);
             __syncwarp();
         }
     }
@@ -1557,9 +1557,9 @@ __global__ void __launch_bounds__(256) cofactor_kernel(const double2* __restrict
                 continue;
             }
             __syncwarp();
-            load_rows(ws, A + s * (int64_t)m * K, K, 1, 0, K - 1, K);
+            load_rows<DIRECT_MAX>(ws, A + s * (int64_t)m * K, K, 1, 0, K - 1, K);
             __syncwarp();
-            cofactors_direct(ws, K);
+            cofactors_direct<DIRECT_MAX>(ws, K);
             if (lane < K) P[s * K + lane] = ws.P[lane];
             __syncwarp();
         }

@@ -2,7 +2,8 @@
 // runs its own stream, so the per-step work (plan, schedules, draw) of many streams proceeds at once
 // and nothing waits on a CTA-wide barrier.  Same algorithm, plan, Gray schedules, all-but-one products,
 // draw rule and uniforms as the CTA form (fock_kernels.cuh); the lanes of the collapsed sum are the
-// warp's 32 / TPL thread groups.  Steps of at most 8 columns sum over the chosen rows directly instead.  Up to 128 modes the marginal's weights stay in registers and one pass
+// warp's 32 / TPL thread groups.  Steps of few columns (WDIRECT) sum over the chosen rows
+// directly instead.  Up to 128 modes the marginal's weights stay in registers and one pass
 // forms the CDF and the pick; beyond, the CDF is formed in 32-mode chunks twice (once for the total, once
 // for the pick) instead of being stored, so any number of modes fits.
 #pragma once
@@ -14,8 +15,13 @@ constexpr int WMAXN = 16;      // photons per stream
 constexpr int WLIN = 128;      // inner schedule length
 constexpr int WMID = 128;      // middle schedule length
 constexpr int WARPS = 8;       // warps (streams in flight) per CTA
+// Steps of at most this many columns are direct: all of the 8-column kernel's, and in the 16-column one as long as the
+// uncollapsed sum in FP64 costs less than the planned step's set-up of about 1 200 instructions (at 10 columns a lane
+// walks 16 terms of 66 FP64 instructions; the mixed form's planned sums are half as dear, so it stops at 9).
+template <int KPW, bool MIXED>
+constexpr int WDIRECT = KPW <= 8 ? 8 : MIXED ? 9 : 10;
 
-// A stream's slice of shared memory: what every step needs, and for kernels beyond DIRECT_MAX columns the plan and
+// A stream's slice of shared memory: what every step needs, and for kernels with planned steps the plan and
 // schedules of the collapsed sum.
 template <int NK>
 struct WarpSmemBase {
@@ -26,7 +32,7 @@ struct WarpSmemBase {
     int cols[NK];
     int64_t cur;
 };
-template <int NK, bool DIRECT = (NK <= DIRECT_MAX)>
+template <int NK, bool DIRECT = (NK <= 8)>
 struct WarpSmemT : WarpSmemBase<NK> {};
 template <int NK>
 struct WarpSmemT<NK, false> : WarpSmemBase<NK> {
@@ -194,7 +200,7 @@ __device__ void sweep_warp_mixed(WS& sm) {
         if (K <= KPv) { CALL; return; }                      \
     }
 
-// A planned step (more than DIRECT_MAX columns).
+// A planned step (more than WDIRECT columns).
 template <int TPL, int KPW, bool MIXED, class WS>
 __device__ void warp_cofactors(WS& sm, int K) {
     if constexpr (MIXED) {
@@ -485,17 +491,17 @@ __device__ void chain_warp(const ChainParams& p, WS& sm, int64_t s) {
             u_mine = chain_uniform((uint64_t)p.seeds[row * p.n_stride + lane], ro);
         }
     }
-    load_rows(sm, A, 1, m, 0, min(kf - 1, DIRECT_MAX - 1), nk);
+    load_rows<KPW>(sm, A, 1, m, 0, min(kf - 1, WDIRECT<KPW, MIXED> - 1), nk);
     __syncwarp();
     for (int k = kf; k <= kend; ++k) {
         const int K1 = k - 1;
-        const bool direct = k <= DIRECT_MAX;
+        const bool direct = k <= WDIRECT<KPW, MIXED>;
         if (K1 == 0) {
             if (lane == 0) sm.P[0] = make_double2(1.0, 0.0);
             __syncwarp();
         } else if (direct) {
-            cofactors_direct(sm, k);
-        } else if constexpr (KPW > DIRECT_MAX) {
+            cofactors_direct<KPW>(sm, k);
+        } else if constexpr (KPW > WDIRECT<KPW, MIXED>) {
             build_groups_warp(sm, K1);
             __syncwarp();
             plan_step(sm, K1, k, 32 / TPL, WLIN, WMID);
@@ -507,13 +513,13 @@ __device__ void chain_warp(const ChainParams& p, WS& sm, int64_t s) {
         const double u = __shfl_sync(0xffffffffu, u_mine, k - 1);
         double* mrow = p.marg ? p.marg + ((size_t)s * p.n_stride + (k - 1)) * p.marg_stride : nullptr;
         const double gap = draw_warp(sm, A, m, k, u, mrow);
-        if constexpr (MIXED && KPW > DIRECT_MAX) {
+        if constexpr (MIXED && (KPW > WDIRECT<KPW, MIXED>)) {
             if (!direct && gap <= guard_band(p, k)) {       // guard band: this step again in FP64
                 warp_cofactors<TPL, KPW, false>(sm, k);
                 draw_warp(sm, A, m, k, u, mrow);
             }
         }
-        if (k < kend && k < DIRECT_MAX) load_rows(sm, A, 1, m, k - 1, k, nk);
+        if (k < kend && k < WDIRECT<KPW, MIXED>) load_rows<KPW>(sm, A, 1, m, k - 1, k, nk);
         __syncwarp();
     }
     for (int j = kf - 1 + lane; j < kend; j += 32) p.rows[s * p.n_stride + j] = sm.rows[j];
