@@ -25,11 +25,16 @@ def pack_instances(U: torch.Tensor, in_modes) -> tuple[torch.Tensor, torch.Tenso
     if U.dim() == 2:
         U = U[None]
     B, m, _ = U.shape
-    idx = torch.as_tensor(list(in_modes), dtype=torch.int64, device=U.device)
-    acol = U.to(torch.complex128)[:, :, idx].transpose(1, 2).contiguous()            # [B, n, m]
-    n = idx.shape[0]
+    modes = [int(j) for j in in_modes]
+    n = len(modes)
     dev = U.device
-    inst_off = torch.arange(B, dtype=torch.int64, device=dev) * (n * m)
+    if n > 0 and modes == list(range(modes[0], modes[0] + n)) and 0 <= modes[0] and modes[-1] < m:
+        cols = U[:, :, modes[0]:modes[0] + n]                # a run of modes: no index tensor to copy over
+    else:
+        cols = U[:, :, torch.tensor(modes, dtype=torch.int64, device=dev)]
+    acol = cols.to(torch.complex128).transpose(1, 2).contiguous()                    # [B, n, m]
+    inst_off = torch.arange(0, B * n * m, n * m, dtype=torch.int64, device=dev) if n * m > 0 else \
+        torch.zeros(B, dtype=torch.int64, device=dev)
     inst_m = torch.full((B,), m, dtype=torch.int32, device=dev)
     inst_n = torch.full((B,), n, dtype=torch.int32, device=dev)
     return acol, inst_off, inst_m, inst_n

@@ -46,10 +46,18 @@ def _cpu_generator(generator):
     return torch.Generator().manual_seed(seed)
 
 
-def _pass_draws(S: int, k: int, generator, dev, max_streams: int):
+def _pass_draws(S: int, k: int, generator, dev, max_streams: int, index: bool = True):
     """sigma [S, k] and per-chunk seeds for one lockstep pass of S streams, drawn chunk by chunk as the
-    reference's `_sample_streams` draws them.  Returns (sigma, seeds [C, k], chunk index [S], offset [S])."""
+    reference's `_sample_streams` draws them.  Returns (sigma, seeds [C, k], chunk index [S], offset [S]); with
+    index=False a pass of one chunk leaves the last two out (the kernels then take row 0 and the stream itself)."""
     gdev = _draw_device(generator, dev)
+    if 0 < S <= max_streams:                     # one chunk: nothing to join
+        sig = torch.argsort(torch.rand(S, k, generator=generator, device=gdev), dim=1).to(dev)
+        seeds = torch.randint(0, 2 ** 31 - 1, (k,), generator=generator, device=gdev).to(dev)[None]
+        if not index:
+            return sig, seeds, None, None
+        return (sig, seeds, torch.zeros(S, dtype=torch.int64, device=dev),
+                torch.arange(S, dtype=torch.int64, device=dev))
     sig, seeds, chunk, off = [], [], [], []
     for ci, c0 in enumerate(range(0, S, max_streams)):
         Sc = min(max_streams, S - c0)
@@ -83,7 +91,7 @@ def sample_chains(U, in_modes, sigma, *, uniforms=None, seeds=None, seed_row=Non
     acol, inst_off, inst_m, inst_n = pack_instances(U, in_modes)
     if split is None:
         split = split_plan(S, n, dev, block_threads, tpl or default_tpl(n, precision), precision)
-    rows, occ, marg = chain(acol, inst_off, inst_m, inst_n, dp, sigma, uniforms=uniforms, seeds=seeds,
+    rows, occ, marg = chain(acol, inst_off, inst_m, inst_n, dp, sigma, m_max=U.shape[1], uniforms=uniforms, seeds=seeds,
                             seed_row=seed_row, rng_off=rng_off, want_occ=True, want_marg=want_marg,
                             precision=precision, block_threads=block_threads, tpl=tpl, grid_ctas=grid_ctas,
                             split=split, mode=mode)
@@ -167,16 +175,21 @@ def fock_sample(U, in_modes, shots, generator=None, algo="auto", multi_min_k1=10
         S = int(reps.sum())
     else:
         S = Bn * int(shots)
-    dp_all = torch.arange(Bn, device=dev, dtype=torch.int64).repeat_interleave(reps if reps is not None else int(shots))
-    occ = torch.zeros(S, m, dtype=torch.int64, device=dev)
+    if Bn == 1:
+        dp_all = torch.zeros(S, dtype=torch.int64, device=dev)
+    else:
+        dp_all = torch.arange(Bn, device=dev, dtype=torch.int64).repeat_interleave(
+            reps if reps is not None else int(shots))
+    occ = None
     if n == 0 or S == 0:
+        occ = torch.zeros(S, m, dtype=torch.int64, device=dev)
         return (occ, torch.arange(S, device=dev, dtype=torch.int64)) if keep_ids else occ
     if uniforms is not None and not (lossless and d is None):
         raise NotImplementedError("uniforms=: lossless, indistinguishable photons only")
     if prefix is not None or avoid is not None:
         return _adaptive(U, in_modes, S, dp_all, generator, max_streams, prefix, avoid, keep_ids, stats,
                          precision, uniforms, block_threads, tpl)
-    plan = plan_chains(U, in_modes, S, dp_all, generator, loss, d, max_streams)
+    plan = plan_chains(U, in_modes, S, dp_all, generator, loss, d, max_streams, _index=False)
     acol, inst_off, inst_m, inst_n = pack_instances(U, in_modes)
     t0 = None
     if stats is not None:
@@ -201,8 +214,8 @@ def fock_sample(U, in_modes, shots, generator=None, algo="auto", multi_min_k1=10
             rows, occ_k, _ = chain(acol, inst_off, inst_m, inst_n, plan.dp, plan.cols, m_max=m, nk=plan.nk, uniforms=u,
                                    seeds=plan.seeds, seed_row=plan.seed_row, rng_off=plan.rng_off, order=plan.order,
                                    want_occ=direct, precision=precision, block_threads=block_threads, tpl=tpl,
-                                   split=split_plan(heavy, n, dev, block_threads,
-                                                    tpl or default_tpl(n, precision), precision))
+                                   split=split_plan(
+                                       heavy, n, dev, block_threads, tpl or default_tpl(n, precision), precision))
             if direct:
                 occ = occ_k
     if stats is not None:
@@ -274,6 +287,7 @@ class ChainPlan:
     (None: all n), seeds [R, n] per-pass-chunk step seeds, seed_row [C] / rng_off [C] the chunk and the local
     stream index of each chain, out_row [C] the output row of each chain (None: chain c is row c), order [C]
     the processing order, single_ids / single_rows the host-routed singleton photons, passes [(k, streams)].
+    seed_row and rng_off are None for one chunk in stream order (fock_sample's own lossless plans).
     """
     S: int
     n: int
@@ -292,7 +306,7 @@ class ChainPlan:
 
 
 def plan_chains(U, in_modes, S: int, dp_all, generator, loss, indist, max_streams: int,
-                _force_general: bool = False) -> ChainPlan:
+                _force_general: bool = False, _index: bool = True) -> ChainPlan:
     """The chains of a call and every host-side draw, consuming `generator` as the reference does
     (sampler.py:146-215): lossless -> one pass of S streams; otherwise the partition on the host generator,
     one pass per surviving count k over the distinct column sets, singletons routed classically last."""
@@ -303,7 +317,7 @@ def plan_chains(U, in_modes, S: int, dp_all, generator, loss, indist, max_stream
     d = as_model(indist)
     lossless = loss is None or float(loss) >= 1.0
     if lossless and d is None:
-        sig, seeds, chunk, off = _pass_draws(S, n, generator, dev, max_streams)
+        sig, seeds, chunk, off = _pass_draws(S, n, generator, dev, max_streams, _index)
         return ChainPlan(S, n, S, dp_all, sig, None, seeds, chunk, off, None, None, None, None, [(n, S)])
     gen = _cpu_generator(generator)
     if d is None and len(set(int(j) for j in in_modes)) == n and not _force_general:

@@ -239,14 +239,13 @@ extern "C" const char* pe_status_string(int status) {
 
 extern "C" int pe_read_status(const void* d_workspace, int* status, int64_t* detail, void* stream) {
     if (!d_workspace || !status) return PE_ERR_ARG;
-    int st = 0;
-    long long det = 0;
+    struct { int status; int pad; long long detail; } w = {0, 0, 0};        // the workspace from byte 8 on
+    static_assert(sizeof(w) == 16, "one copy of both words");
     cudaStream_t s = (cudaStream_t)stream;
-    PE_CUDA_TRY(cudaMemcpyAsync(&st, (const char*)d_workspace + 8, sizeof(int), cudaMemcpyDeviceToHost, s));
-    PE_CUDA_TRY(cudaMemcpyAsync(&det, (const char*)d_workspace + 16, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    PE_CUDA_TRY(cudaMemcpyAsync(&w, (const char*)d_workspace + 8, sizeof(w), cudaMemcpyDeviceToHost, s));
     PE_CUDA_TRY(cudaStreamSynchronize(s));
-    *status = st;
-    if (detail) *detail = (int64_t)det;
+    *status = w.status;
+    if (detail) *detail = (int64_t)w.detail;
     return PE_OK;
 }
 
