@@ -154,6 +154,44 @@ def split_plan(heavy_streams: int, n: int, device, block_threads: int = 0, tpl: 
     return (k, nch) if k <= n else None
 
 
+# Blocks of four terms per Gray lane below which a CTA of a split step costs more in planning its share than the
+# share itself, and the waves worth filling up to 26 photons (pair sweep; measured, FP64 ms: n = 20, m = 400, 32
+# streams 64 -> 16 CTAs each 0.74 -> 0.57; n = 24, m = 48, 512 streams 16 -> 8 CTAs 20.3 -> 17.8, 64 streams 128 -> 64
+# CTAs 5.1 -> 4.0; n = 22, m = 88, 100 streams 32 -> 16 CTAs 2.78 -> 2.34; one stream of n = 20 keeps its 64).
+PAIR_BLOCKS_PER_LANE = 64
+PAIR_FILL, PAIR_FILL_LONG = 5, 8
+
+
+def split_shape(heavy_streams: int, n: int, device, block_threads: int = 0, tpl: int = 2, precision: str = "f64"):
+    """split_plan for a launch whose streams all have n photons, with fewer CTAs per stream where the pair sweep runs
+    its steps (up to 32 photons, FP64 and mixed forms): a step's work shrank but not what a CTA spends on its plan,
+    so a stream gets no more CTAs than fill PAIR_FILL waves (PAIR_FILL_LONG at 24-26 photons), nor so many that a
+    lane of the last step walks fewer than PAIR_BLOCKS_PER_LANE blocks, unless SMs would stay idle; k_split is the
+    first step with eight blocks per lane (one for fewer than 16 streams)."""
+    plan = split_plan(heavy_streams, n, device, block_threads, tpl, precision)
+    if plan is None or n > N.PE_MIXED_MAX_PHOTONS or precision == "compensated" or n < 17:
+        return plan
+    dev = torch.device(device)
+    block = block_threads or DEFAULT_BLOCK
+    slots = _split_slots(dev.index if dev.index is not None else torch.cuda.current_device(), precision, n, block,
+                         tpl or default_tpl(n, precision))
+    lanes = block // (2 if n <= 20 else 4) * (2 if precision == "mixed" else 1)
+    blocks = 1 << (n - 4)
+    k, nch = plan
+    if n <= 26:
+        waves = PAIR_FILL if n < 24 else PAIR_FILL_LONG
+        while nch > 2 and heavy_streams * (nch // 2) >= waves * slots:
+            nch //= 2
+    while nch > 2 and blocks < PAIR_BLOCKS_PER_LANE * lanes * nch and heavy_streams * nch > slots:
+        nch //= 2
+    per_lane = 8 if heavy_streams >= 16 else 1
+    k = max(PAIR_MIN_COLUMNS, 4)
+    while k < n and (1 << (k - 4)) < per_lane * nch * lanes:
+        k += 1
+    return k, nch
+
+
+PAIR_MIN_COLUMNS = 9         # the pair sweep's first step (fock_kernels.cuh PAIRS_MIN)
 WARP_MAX_PHOTONS = 16
 
 

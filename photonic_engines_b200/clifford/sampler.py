@@ -26,7 +26,8 @@ import torch
 
 from .. import _native as N
 from ..imperfections import as_model, draw_fates, group_fates, route_lone_photons
-from .kernels import chain, chain_adaptive, chain_tiers, default_tpl, pack_instances, split_plan, tier_plan
+from .kernels import (chain, chain_adaptive, chain_tiers, default_tpl, pack_instances, split_plan, split_shape,
+                      tier_plan)
 from .prefix import prefix_order
 
 BACKENDS = ("b200", "triton", "cuda", "exq")
@@ -90,7 +91,7 @@ def sample_chains(U, in_modes, sigma, *, uniforms=None, seeds=None, seed_row=Non
         dp = torch.zeros(S, dtype=torch.int64, device=dev)
     acol, inst_off, inst_m, inst_n = pack_instances(U, in_modes)
     if split is None:
-        split = split_plan(S, n, dev, block_threads, tpl or default_tpl(n, precision), precision)
+        split = split_shape(S, n, dev, block_threads, tpl or default_tpl(n, precision), precision)
     rows, occ, marg = chain(acol, inst_off, inst_m, inst_n, dp, sigma, m_max=U.shape[1], uniforms=uniforms, seeds=seeds,
                             seed_row=seed_row, rng_off=rng_off, want_occ=True, want_marg=want_marg,
                             precision=precision, block_threads=block_threads, tpl=tpl, grid_ctas=grid_ctas,
@@ -214,7 +215,7 @@ def fock_sample(U, in_modes, shots, generator=None, algo="auto", multi_min_k1=10
             rows, occ_k, _ = chain(acol, inst_off, inst_m, inst_n, plan.dp, plan.cols, m_max=m, nk=plan.nk, uniforms=u,
                                    seeds=plan.seeds, seed_row=plan.seed_row, rng_off=plan.rng_off, order=plan.order,
                                    want_occ=direct, precision=precision, block_threads=block_threads, tpl=tpl,
-                                   split=split_plan(
+                                   split=(split_shape if plan.nk is None else split_plan)(
                                        heavy, n, dev, block_threads, tpl or default_tpl(n, precision), precision))
             if direct:
                 occ = occ_k

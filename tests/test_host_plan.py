@@ -135,3 +135,22 @@ def test_tier_plan_cuts_the_longest_first_queue(monkeypatch):
     t = K.tier_plan({12: 100, 7: 50}, 12, "f64", "cuda:0")
     assert t == [(0, 150, 12, 1, None)]                          # one tier: the plain launch runs it
     assert K.tier_plan({}, 30, "f64", "cuda:0") == []
+
+
+@pytest.mark.parametrize(("heavy", "n", "expect"), [
+    (1, 20, (16, 64)),              # one stream keeps its CTAs: the other SMs are idle
+    (32, 20, (17, 16)),             # 64 blocks per lane of the last step, eight at the first split one
+    (512, 24, (15, 8)), (64, 24, (18, 64)),   # eight waves
+    (200, 28, (18, 64)),            # long chains keep split_plan's CTAs
+    (200, 40, (17, 64)),            # past the pair sweep: split_plan's own
+    (3, 6, None),
+])
+def test_split_shape_gives_pair_sweep_steps_fewer_ctas(monkeypatch, heavy, n, expect):
+    """The launch shape of lossless calls on the CPU, resident CTAs stubbed (296)."""
+    from photonic_engines_b200.clifford import kernels as K
+    monkeypatch.setattr(K, "_split_slots", lambda *a: 296)
+    got = K.split_shape(heavy, n, "cuda:0", 128, K.default_tpl(n, "f64"), "f64")
+    if n == 40:
+        assert got == K.split_plan(heavy, n, "cuda:0", 128, K.default_tpl(n, "f64"), "f64")
+    else:
+        assert got == expect
