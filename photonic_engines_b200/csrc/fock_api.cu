@@ -70,11 +70,13 @@ void* find_cofactor_kernel(int mixed, int tpl, int kpm) {
     return (!prec_ok(mixed) || ti < 0 || ki < 0) ? nullptr : g_cof[mixed][ti][ki];
 }
 
-// Threads per Gray lane when the caller passes 0 (measured at m = 400, 2 000 streams, and at m = 2n for
+// Threads per Gray lane when the caller passes 0 (term by term, measured at m = 400, 2 000 streams, and at m = 2n for
 // 21-32 photons): one-thread lanes up to 8 columns, and for FP64 and mixed chains of 17-20 photons (no
 // exchange of partial products; those variants run 128-thread CTAs with 255 registers: n = 20, m = 400,
 // FP64 18.4 against 21.0 ms with two-thread lanes, mixed 12.8 against 13.4 ms); two-thread lanes beyond
-// (at 24-40 columns compiled for 128-thread CTAs with 255 registers), four-thread lanes at 48-64.
+// (at 24-40 columns compiled for 128-thread CTAs with 255 registers), four-thread lanes at 48-64.  The lane width
+// names the compiled variant and rules its term-by-term sweep; the pair sweep inside the 255-register variants has
+// lanes of its own (fock_pairs.cuh), which the times above do not include.
 static int default_tpl(int kpm, int precision) {
     if (kpm <= 8) return 1;
     if (precision != PE_PRECISION_COMPENSATED && kpm == 20) return 1;

@@ -1066,12 +1066,16 @@ constexpr int PAIRS_LIN32 = 128;       // mixed form: FP32 inner blocks of at mo
 constexpr int PAIRS_ONES32 = 6;
 template <int TPL, int KPM>
 __host__ __device__ constexpr bool has_pairs() {
-    return PE_MAXT * PE_MINB <= 384 && TPL <= 2 && KPM >= PAIRS_MIN && KPM <= NARROW;
+    return PE_MAXT * PE_MINB <= 256 && TPL <= 2 && KPM >= PAIRS_MIN && KPM <= NARROW;
 }
-#ifndef PE_PAIR4
-#define PE_PAIR4 20
-#endif
-__host__ __device__ constexpr int pair_tpl(int K) { return K <= PE_PAIR4 ? 2 : 4; }
+__host__ __device__ constexpr int pair_tpl(int K) { return K <= 20 ? 2 : 4; }
+// Columns of a pair step's tier: multiples of four, and 18 in FP64 (nine columns per thread, the odd one an item of
+// its own: without the padding to 20 and its spills, cofactors at 18 columns 4.8 -> 4.3 ms for 4 736 blocks, n = 18,
+// m = 324, 4 000 streams 7.66 -> 7.14 ms, n = 20, m = 400, 2 000 streams 13.88 -> 13.68; 10 and 14 columns gained
+// nothing over 12 and 16).
+__host__ __device__ constexpr int pair_tier(int K, int prec) {
+    return prec == PREC_F64 && (K == 17 || K == 18) ? 18 : (K + 3) / 4 * 4;
+}
 
 // Tiers the term-by-term FP64 sweep is compiled for: all of them, but where the pair sweep runs a tier only
 // crowded steps (fewer than two modes chosen once) are left, and the kernel's last tier serves those.
@@ -1109,17 +1113,19 @@ __device__ void dispatch_mixed(SM& sm, int K) {
 
 namespace pe {
 
-#define PE_PTIER(KPv)                                                                            \
-    if constexpr (KPM >= KPv) {                                                                  \
-        if (K <= KPv) {                                                                          \
-            if constexpr (PREC == PREC_MIXED) sweep_pairs_mixed<KPv / pair_tpl(KPv), pair_tpl(KPv) / 2, SM>(); \
-            else sweep_pairs_f64<KPv / pair_tpl(KPv), pair_tpl(KPv), SM>();                        \
-            return;                                                                              \
-        }                                                                                        \
+#define PE_PTIER(KPv)                                                                              \
+    if constexpr (KPM >= KPv && pair_tier(KPv, PREC) == KPv) {                                     \
+        if (K <= KPv) {                                                                            \
+            if constexpr (PREC == PREC_MIXED)                                                      \
+                sweep_pairs_mixed<KPv / pair_tpl(KPv), pair_tpl(KPv) / 2, SM>();                   \
+            else                                                                                   \
+                sweep_pairs_f64<KPv / pair_tpl(KPv), pair_tpl(KPv), SM>();                         \
+            return;                                                                                \
+        }                                                                                          \
     }
 template <int KPM, int PREC, class SM>
 __device__ void dispatch_pairs(SM& sm, int K) {
-    PE_PTIER(12) PE_PTIER(16) PE_PTIER(20) PE_PTIER(24) PE_PTIER(28) PE_PTIER(32)
+    PE_PTIER(12) PE_PTIER(16) PE_PTIER(18) PE_PTIER(20) PE_PTIER(24) PE_PTIER(28) PE_PTIER(32)
 }
 
 // One cofactor step of the stream held in shared memory (K1 >= 1): plan, prepare, sweep.  PREC: 0 FP64,
@@ -1128,7 +1134,7 @@ template <int TPL, int KPM, int PREC, class SM>
 __device__ __forceinline__ void cofactor_step(SM& sm, const double2* A, int64_t rs, int64_t cs, int K1, int K) {
     constexpr bool MIXED = PREC == PREC_MIXED;
     constexpr bool PAIRS = PREC != PREC_COMP && has_pairs<TPL, KPM>();
-    const int kp = (K + 3) / 4 * 4, ptl = pair_tpl(K) == 2 ? 1 : 2, pkh = kp >> ptl;
+    const int ptl = pair_tpl(K) == 2 ? 1 : 2, pkh = pair_tier(K, PREC) >> ptl;
     if (threadIdx.x < 32)
         plan_step(sm, K1, K, blockDim.x / TPL * sm.lane_mult, MIXED ? MIXED_LIN : LIN_MAX, MID_MAX,
                   PAIRS && K >= PAIRS_MIN ? (blockDim.x >> (MIXED ? ptl - 1 : ptl)) * sm.lane_mult : 0,
@@ -1137,7 +1143,7 @@ __device__ __forceinline__ void cofactor_step(SM& sm, const double2* A, int64_t 
     bool pairs = false;
     if constexpr (PAIRS) pairs = sm.plan.pairs;
     // paired FP32 sweeps (mixed form, 1- and 2-thread lanes): columns per thread of the dispatched tier
-    const int kh = !MIXED ? 0 : pairs ? 2 * pkh : (PE_PAIR32 && TPL <= 2) ? kp / TPL : 0;
+    const int kh = !MIXED ? 0 : pairs ? 2 * pkh : (PE_PAIR32 && TPL <= 2) ? (K + 3) / 4 * 4 / TPL : 0;
     prepare_step(sm, A, rs, cs, MIXED, kh, pairs && !MIXED ? pkh : 0, ptl);
     __syncthreads();
     if constexpr (PREC == PREC_COMP) {

@@ -35,7 +35,7 @@ def _check(K: int, rows: np.ndarray, block: int = 128, tpl: int | None = None):
         assert np.abs(P[s] - ref).max() <= tol * np.abs(ref).max(), (K, rows.tolist(), s)
 
 
-@pytest.mark.parametrize("K", [9, 10, 11, 12, 13, 16, 17, 20])
+@pytest.mark.parametrize("K", [9, 10, 11, 12, 13, 16, 17, 18, 19, 20])
 def test_tier_edges_with_distinct_rows(K):
     _check(K, _rows(K - 1, K - 1, 2))
 
