@@ -32,7 +32,10 @@ def pack_instances(U: torch.Tensor, in_modes) -> tuple[torch.Tensor, torch.Tenso
         cols = U[:, :, modes[0]:modes[0] + n]                # a run of modes: no index tensor to copy over
     else:
         cols = U[:, :, torch.tensor(modes, dtype=torch.int64, device=dev)]
-    acol = cols.to(torch.complex128).transpose(1, 2).contiguous()                    # [B, n, m]
+    # a copy of its own whatever U is: a run's slice may already lie in this layout (U.mH, U.mT), and then
+    # contiguous() would hand back U's memory, with its conjugation flag
+    acol = torch.empty(B, n, m, dtype=torch.complex128, device=dev)
+    acol.copy_(cols.transpose(1, 2))
     inst_off = torch.arange(0, B * n * m, n * m, dtype=torch.int64, device=dev) if n * m > 0 else \
         torch.zeros(B, dtype=torch.int64, device=dev)
     inst_m = torch.full((B,), m, dtype=torch.int32, device=dev)
