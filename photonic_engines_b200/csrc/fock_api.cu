@@ -251,16 +251,36 @@ extern "C" int pe_read_status(const void* d_workspace, int* status, int64_t* det
     return PE_OK;
 }
 
-static int launch_prepare(void* fn, int block, size_t smem, int* grid_per_sm) {
-    PE_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+// Resident CTAs per SM of a kernel at `smem` bytes.  A kernel's only attribute is a constant (it may use all of the
+// opt-in limit `cap`; the kernels have no static shared memory), so calls of other sizes, earlier ones or those of
+// other host threads, change neither what a launch may use nor what the occupancy query answers.
+static int launch_prepare(void* fn, int block, size_t smem, int cap, int* grid_per_sm) {
+    PE_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
     int occ = 0;
     PE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, block, smem));
     if (occ < 1) return PE_ERR_SIZE;
-    // the rest of the SM's 228 KB stays L1 (register spills, the instance's columns); a CTA holds 1 KB beside its own
-    const int carve = (int)((100 * (size_t)occ * (smem + 1024) + 228 * 1024 - 1) / (228 * 1024));
-    PE_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, carve < 100 ? carve : 100));
     *grid_per_sm = occ;
     return PE_OK;
+}
+
+// One launch that asks for no more shared memory than its per_sm resident CTAs hold: the rest of the SM's 228 KB stays
+// L1 (register spills, the instance's columns); a CTA holds 1 KB beside its own.  The request goes with the launch:
+// as an attribute of the function it outlived the call and lowered the occupancy that the next one was told (n = 18,
+// m = 5 000, 2 000 streams: 9.9 instead of 6.6 ms after a call with m = 300, and 5.1 instead of 3.8 ms the other way round).
+static cudaError_t launch_kernel(void* fn, int64_t grid, int block, void** args, size_t smem, int per_sm,
+                                 cudaStream_t stream) {
+    const unsigned carve = (unsigned)((100 * (size_t)per_sm * (smem + 1024) + 228 * 1024 - 1) / (228 * 1024));
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr.val.sharedMemCarveout = carve < 100u ? carve : 100u;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
 // Checks, variant lookup and launches shared by the chain entry points.  k_split = 0: the whole chain in
@@ -324,7 +344,7 @@ static int chain_launch(int precision, const double* d_acol, const int64_t* d_in
     if (S == 0) return PE_OK;
     const int klast = (k_last > 0 && k_last < n_stride) ? k_last : n_stride;
     int per_sm = 0;
-    int rc = launch_prepare(fn, block, smem, &per_sm);
+    int rc = launch_prepare(fn, block, smem, cap, &per_sm);
     if (rc != PE_OK) return rc;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -355,23 +375,25 @@ static int chain_launch(int precision, const double* d_acol, const int64_t* d_in
     p.k_stop = split ? (k_split - 1 < klast ? k_split - 1 : klast) : (k_last > 0 ? klast : 0);
     p.split_cap = (split && d_qrange) ? nq : -1;
     void* args[] = {&p};
-    PE_CUDA_TRY(cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(block), args, smem, st));
+    PE_CUDA_TRY(launch_kernel(fn, grid, block, args, smem, per_sm, st));
     if (!split) return PE_OK;
     // the mixed form's guard band: flagged streams redo the step with the FP64 kernels (second pass)
     const int npass = precision != PE_PRECISION_F64 ? 2 : 1;
     void* fpart[2] = {find_split_partial_kernel(precision, tpl, kpm), find_split_partial_kernel(PE_PRECISION_F64, tpl, kpm)};
     void* fdraw[2] = {find_split_draw_kernel(precision, tpl, kpm), find_split_draw_kernel(PE_PRECISION_F64, tpl, kpm)};
     int64_t gpart[2], gdraw[2];
+    int per_part[2], per_draw[2];
+    size_t spart[2], sdraw[2];
     const int64_t items = nq * (int64_t)nch;
     for (int q = 0; q < npass; ++q) {
         if (!fpart[q] || !fdraw[q]) return PE_ERR_SIZE;
-        int per_part = 0, per_draw = 0;
         const int pq = q == 0 ? precision : PE_PRECISION_F64;
-        const size_t sdraw = cta_smem_bytes(kpm, pq, m_max);
-        if ((rc = launch_prepare(fpart[q], block, cta_smem_bytes(kpm, pq, 0), &per_part)) != PE_OK) return rc;
-        if ((rc = launch_prepare(fdraw[q], block, sdraw, &per_draw)) != PE_OK) return rc;
-        gpart[q] = items < (int64_t)sms * per_part ? items : (int64_t)sms * per_part;
-        gdraw[q] = nq < (int64_t)sms * per_draw ? nq : (int64_t)sms * per_draw;
+        spart[q] = cta_smem_bytes(kpm, pq, 0);
+        sdraw[q] = cta_smem_bytes(kpm, pq, m_max);
+        if ((rc = launch_prepare(fpart[q], block, spart[q], cap, &per_part[q])) != PE_OK) return rc;
+        if ((rc = launch_prepare(fdraw[q], block, sdraw[q], cap, &per_draw[q])) != PE_OK) return rc;
+        gpart[q] = items < (int64_t)sms * per_part[q] ? items : (int64_t)sms * per_part[q];
+        gdraw[q] = nq < (int64_t)sms * per_draw[q] ? nq : (int64_t)sms * per_draw[q];
     }
     SplitParams sp;
     sp.c = p;
@@ -385,11 +407,8 @@ static int chain_launch(int precision, const double* d_acol, const int64_t* d_in
         sp.k = k;
         for (int q = 0; q < npass; ++q) {
             sp.pass = q;
-            const int pq = q == 0 ? precision : PE_PRECISION_F64;
-            PE_CUDA_TRY(cudaLaunchKernel(fpart[q], dim3((unsigned)gpart[q]), dim3(block), sargs,
-                                         cta_smem_bytes(kpm, pq, 0), st));
-            PE_CUDA_TRY(cudaLaunchKernel(fdraw[q], dim3((unsigned)gdraw[q]), dim3(block), sargs,
-                                         cta_smem_bytes(kpm, pq, m_max), st));
+            PE_CUDA_TRY(launch_kernel(fpart[q], gpart[q], block, sargs, spart[q], per_part[q], st));
+            PE_CUDA_TRY(launch_kernel(fdraw[q], gdraw[q], block, sargs, sdraw[q], per_draw[q], st));
         }
     }
     return PE_OK;
@@ -551,12 +570,14 @@ extern "C" int pe_cofactors_rows(int precision, const double* d_a, const int64_t
     if (bmax < 32) return PE_ERR_CUDA;
     const int block = block_threads ? block_threads : (bmax < 256 ? bmax : 256);
     if (block < 32 || block > 256 || block > bmax || (block & 31) || block < K) return PE_ERR_ARG;
+    const int cap = max_smem_optin();
+    if (cap <= 0) return PE_ERR_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
     PE_CUDA_TRY(cudaMemsetAsync(d_workspace, 0, WS_BYTES, st));
     if (S == 0) return PE_OK;
     const size_t smem = cta_smem_bytes(kpm, precision, 0);
     int per_sm = 0;
-    int rc = launch_prepare(fn, block, smem, &per_sm);
+    int rc = launch_prepare(fn, block, smem, cap, &per_sm);
     if (rc != PE_OK) return rc;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -568,7 +589,7 @@ extern "C" int pe_cofactors_rows(int precision, const double* d_a, const int64_t
     int* status = (int*)((char*)d_workspace + 8);
     long long* detail = (long long*)((char*)d_workspace + 16);
     void* args[] = {(void*)&a, (void*)&d_rows, (void*)&S, (void*)&m, (void*)&K, (void*)&pp, (void*)&status, (void*)&detail};
-    PE_CUDA_TRY(cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(block), args, smem, st));
+    PE_CUDA_TRY(launch_kernel(fn, grid, block, args, smem, per_sm, st));
     return PE_OK;
 }
 
@@ -589,7 +610,9 @@ extern "C" int pe_split_slots(int precision, int n_stride, int block_threads, in
     const int block = block_threads ? block_threads : (bmax < 128 ? bmax : 128);
     if (block < 32 || block > 256 || block > bmax || (block & 31)) return PE_ERR_ARG;
     int per_sm = 0, dev = 0, sms = 0;
-    const int rc = launch_prepare(fn, block, cta_smem_bytes(kpm, precision, 0), &per_sm);
+    const int cap = max_smem_optin();
+    if (cap <= 0) return PE_ERR_CUDA;
+    const int rc = launch_prepare(fn, block, cta_smem_bytes(kpm, precision, 0), cap, &per_sm);
     if (rc != PE_OK) return rc;
     PE_CUDA_TRY(cudaGetDevice(&dev));
     PE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
