@@ -1181,7 +1181,8 @@ __device__ __forceinline__ void redo_step_f64(SM& sm, const double2* A, int64_t 
 // ---------------------------------------------------------------------------------------- draw
 // Marginal over the m output modes, FP64 block scan (contiguous chunk per thread, warp scan, warps
 // in order), then idx = min(#{rho : cw_rho < u * tot}, m - 1) with tot = cw[m - 1]
-// (cofactors_triton.py:298-308).  All threads return the pick, and (GAP) the gap min |cw - u tot| / tot; thread 0 has
+// (cofactors_triton.py:298-308).  Every thread forms tot itself, in the order of its owner (at most m / threads + 1
+// additions of weights in shared memory) rather than wait for it at a fourth barrier.  All threads return the pick, and (GAP) the gap min |cw - u tot| / tot; thread 0 has
 // written it to sm.rows and warp 0 (groups) added it to the groups, with no barrier after that.  Three barriers: short
 // steps are bound by them and by the latencies between them.
 template <bool GAP, class SM>
@@ -1235,15 +1236,23 @@ static __device__ int draw_step(SM& sm, double* __restrict__ wgt, const double2*
     }
     double excl = __shfl_up_sync(0xffffffffu, x, 1);
     if (lid == 0) excl = 0.0;
+    const int tl = (m - 1) / C, wl = tl >> 5;           // the thread that owns mode m - 1, and its warp
     if (lid == 31) sm.scan[wid] = x;
+    if (tid == tl) sm.last_excl = excl;
     __syncthreads();
-    double E = 0.0, tot = 0.0;
+    double E = 0.0, tot = 0.0;                          // weights below the thread's modes, and below thread tl's
+    {
+        double below = 0.0;
 #pragma unroll
-    for (int w = 0; w < MAX_WARPS; ++w) {
-        if (w == wid) E = tot;
-        if (w < nw) tot += sm.scan[w];
+        for (int w = 0; w < MAX_WARPS; ++w) {
+            if (w == wid) E = below;
+            if (w == wl) tot = below;
+            if (w < nw) below += sm.scan[w];
+        }
     }
     E += excl;
+    tot += sm.last_excl;
+    for (int i = tl * C; i < m; ++i) tot += wgt[i];     // cw[m - 1] as thread tl forms it
     const double target = u * tot;
     int cnt = 0;
     double gmin = 1.0e300;
