@@ -277,8 +277,8 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
             const unsigned eq = __ballot_sync(full, take);
             if (take) {
                 const int r = na + __popc(eq & below);
-                pl.sortR[r] = R[q];
-                pl.sortG[r] = lane + 32 * q;
+                pl.sortR[r] = (unsigned char)R[q];
+                pl.sortG[r] = (unsigned char)(lane + 32 * q);
             }
             na += __popc(eq);
             rem[q] &= ~eq;
@@ -360,8 +360,8 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
             pl.R[kd] = (int)rv[q];
             pl.M[kd] = mp[q];
             pl.drow[kd] = sm.grow[gp[q]];
-            if (p >= nhi && p < nhi + nin) pl.Pin[kd] = pin[q];
-            if (p >= nhi + nin && p < nhi + nin + nmid) pl.Pmid[kd - nin] = pmid[q];
+            if (p >= nhi && p < nhi + nin) pl.Pin[kd] = (unsigned short)pin[q];
+            if (p >= nhi + nin && p < nhi + nin + nmid) pl.Pmid[kd - nin] = (unsigned short)pmid[q];
         }
         const int g = lane + 32 * q;                   // fixed digits: after the active ones, in group order
         const bool fixed = g < D && !active[q] && g != gu && g != gv;
@@ -397,7 +397,7 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
 // ones: every digit has radix 2 and multiplicity 1, so the digits are the bits of the Gray code of t and the
 // weight its parity.  vend (optional): the digit values at t.
 template <class PL>
-static __device__ __forceinline__ unsigned char gray_entry(const PL& pl, int d0, int nd, const int* Pp, int t,
+static __device__ __forceinline__ unsigned char gray_entry(const PL& pl, int d0, int nd, const unsigned short* Pp, int t,
                                                           double* w_out, unsigned char* vend, bool ones) {
     if (ones) {
         const int g = t ^ (t >> 1);
