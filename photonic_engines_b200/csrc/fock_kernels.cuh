@@ -1236,12 +1236,12 @@ static __device__ int draw_step(SM& sm, double* __restrict__ wgt, const double2*
     }
     double excl = __shfl_up_sync(0xffffffffu, x, 1);
     if (lid == 0) excl = 0.0;
-    const int tl = (m - 1) / C, wl = tl >> 5;           // the thread that owns mode m - 1, and its warp
     if (lid == 31) sm.scan[wid] = x;
-    if (tid == tl) sm.last_excl = excl;
+    if (lo < m && hi == m) { sm.last_excl = excl; sm.last_lo = lo; sm.last_warp = wid; }      // the owner of mode m - 1
     __syncthreads();
-    double E = 0.0, tot = 0.0;                          // weights below the thread's modes, and below thread tl's
+    double E = 0.0, tot = 0.0;                          // weights below the thread's modes, and below the owner's
     {
+        const int wl = sm.last_warp;
         double below = 0.0;
 #pragma unroll
         for (int w = 0; w < MAX_WARPS; ++w) {
@@ -1252,7 +1252,8 @@ static __device__ int draw_step(SM& sm, double* __restrict__ wgt, const double2*
     }
     E += excl;
     tot += sm.last_excl;
-    for (int i = tl * C; i < m; ++i) tot += wgt[i];     // cw[m - 1] as thread tl forms it
+#pragma unroll 4
+    for (int i = sm.last_lo; i < m; ++i) tot += wgt[i]; // cw[m - 1] as its owner forms it
     const double target = u * tot;
     int cnt = 0;
     double gmin = 1.0e300;

@@ -112,7 +112,8 @@ struct SmemT {
     unsigned char tab_fm[MID_MAX]; // transition into middle index: middle digit | 0x80 when -2 b
     double2 red[MAX_WARPS][NK];  // cross-warp reduction
     double scan[MAX_WARPS];
-    double last_excl;            // the draw: weights below mode m - 1's thread, within its warp
+    double last_excl;            // the draw: weights below those of mode m - 1's thread, within its warp,
+    int last_lo, last_warp;      // its first mode, and its warp
     long long gap_bits;          // the draw: smallest distance of the cumulative weights to u tot (bits of a double)
     int below;                   // and how many of them lie below it
     double u[NK];                // the steps' uniforms
