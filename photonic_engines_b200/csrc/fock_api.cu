@@ -31,14 +31,16 @@ static void* g_split_partial[N_PREC][3][N_KPM];
 static void* g_split_draw[N_PREC][3][N_KPM];
 static void* g_warp[N_PREC][3][N_KPM];
 static size_t g_warp_slice[N_PREC][3][N_KPM];
+static size_t g_pair_tables[N_PREC][3][N_KPM];
 static bool prec_ok(int p) { return p >= 0 && p < N_PREC; }
 
 void register_variant(int mixed, int tpl, int kpm, void* chain_kernel, void* cofactor_kernel, void* split_partial,
-                      void* split_draw, void* warp_kernel, size_t warp_slice_bytes) {
+                      void* split_draw, void* warp_kernel, size_t warp_slice_bytes, size_t pair_table_bytes) {
     const int ti = tpl_index(tpl), ki = kpm_index(kpm);
     if (!prec_ok(mixed) || ti < 0 || ki < 0) return;
     g_warp[mixed][ti][ki] = warp_kernel;
     g_warp_slice[mixed][ti][ki] = warp_slice_bytes;
+    g_pair_tables[mixed][ti][ki] = pair_table_bytes;
     g_chain[mixed][ti][ki] = chain_kernel;
     g_cof[mixed][ti][ki] = cofactor_kernel;
     g_split_partial[mixed][ti][ki] = split_partial;
@@ -51,6 +53,10 @@ void* find_split_partial_kernel(int mixed, int tpl, int kpm) {
 void* find_warp_kernel(int mixed, int tpl, int kpm) {
     const int ti = tpl_index(tpl), ki = kpm_index(kpm);
     return (!prec_ok(mixed) || ti < 0 || ki < 0) ? nullptr : g_warp[mixed][ti][ki];
+}
+size_t pair_table_bytes(int mixed, int tpl, int kpm) {
+    const int ti = tpl_index(tpl), ki = kpm_index(kpm);
+    return (!prec_ok(mixed) || ti < 0 || ki < 0) ? 0 : g_pair_tables[mixed][ti][ki];
 }
 size_t warp_smem_bytes(int mixed, int tpl, int kpm, int warps) {
     const int ti = tpl_index(tpl), ki = kpm_index(kpm);
@@ -193,11 +199,9 @@ __global__ void __launch_bounds__(1024) avoid_update_kernel(AvoidParams a) {
     }
 }
 
-// Dynamic shared memory of a CTA: the tier's layout, then `weights` draw weights (0: a kernel without a draw); the
-// FP64 and mixed tiers up to 32 columns lay the pair sweep's tables over the weights.
-static size_t cta_smem_bytes(int kpm, int prec, int weights) {
-    const size_t tables = kpm > NARROW ? 0 : prec == PE_PRECISION_F64 ? sizeof(PairTables<NARROW>)
-                        : prec == PE_PRECISION_MIXED ? sizeof(PairTables32<NARROW>) : 0;
+// Dynamic shared memory of a CTA: the tier's layout, then `weights` draw weights (0: a kernel without a draw) and over
+// them `tables` bytes of the pair sweep's tables (0: a variant or a kernel without that sweep).
+static size_t cta_smem_bytes(int kpm, int prec, int weights, size_t tables) {
     const size_t w = (size_t)weights * sizeof(double);
     return smem_fixed_bytes_for(kpm, prec) + (w > tables ? w : tables);
 }
@@ -335,7 +339,7 @@ static int chain_launch(int precision, const double* d_acol, const int64_t* d_in
     if (block < 32 || block > 256 || block > bmax || (block & 31)) return PE_ERR_ARG;
     if (!warp_mode && block < ncols) return PE_ERR_ARG;
     const size_t smem = warp_mode ? warp_smem_bytes(precision, tpl, kpm, block / 32)
-                                  : cta_smem_bytes(kpm, precision, m_max);
+                                  : cta_smem_bytes(kpm, precision, m_max, pair_table_bytes(precision, tpl, kpm));
     const int cap = max_smem_optin();
     if (cap <= 0) return PE_ERR_CUDA;
     if (smem > (size_t)cap) return PE_ERR_SIZE;
@@ -388,8 +392,8 @@ static int chain_launch(int precision, const double* d_acol, const int64_t* d_in
     for (int q = 0; q < npass; ++q) {
         if (!fpart[q] || !fdraw[q]) return PE_ERR_SIZE;
         const int pq = q == 0 ? precision : PE_PRECISION_F64;
-        spart[q] = cta_smem_bytes(kpm, pq, 0);
-        sdraw[q] = cta_smem_bytes(kpm, pq, m_max);
+        spart[q] = cta_smem_bytes(kpm, pq, 0, pair_table_bytes(pq, tpl, kpm));
+        sdraw[q] = cta_smem_bytes(kpm, pq, m_max, 0);
         if ((rc = launch_prepare(fpart[q], block, spart[q], cap, &per_part[q])) != PE_OK) return rc;
         if ((rc = launch_prepare(fdraw[q], block, sdraw[q], cap, &per_draw[q])) != PE_OK) return rc;
         gpart[q] = items < (int64_t)sms * per_part[q] ? items : (int64_t)sms * per_part[q];
@@ -575,7 +579,7 @@ extern "C" int pe_cofactors_rows(int precision, const double* d_a, const int64_t
     cudaStream_t st = (cudaStream_t)stream;
     PE_CUDA_TRY(cudaMemsetAsync(d_workspace, 0, WS_BYTES, st));
     if (S == 0) return PE_OK;
-    const size_t smem = cta_smem_bytes(kpm, precision, 0);
+    const size_t smem = cta_smem_bytes(kpm, precision, 0, pair_table_bytes(precision, tpl, kpm));
     int per_sm = 0;
     int rc = launch_prepare(fn, block, smem, cap, &per_sm);
     if (rc != PE_OK) return rc;
@@ -612,7 +616,8 @@ extern "C" int pe_split_slots(int precision, int n_stride, int block_threads, in
     int per_sm = 0, dev = 0, sms = 0;
     const int cap = max_smem_optin();
     if (cap <= 0) return PE_ERR_CUDA;
-    const int rc = launch_prepare(fn, block, cta_smem_bytes(kpm, precision, 0), cap, &per_sm);
+    const int rc = launch_prepare(fn, block, cta_smem_bytes(kpm, precision, 0, pair_table_bytes(precision, tpl, kpm)), cap,
+                                  &per_sm);
     if (rc != PE_OK) return rc;
     PE_CUDA_TRY(cudaGetDevice(&dev));
     PE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

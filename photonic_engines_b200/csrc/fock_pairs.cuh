@@ -563,4 +563,11 @@ __device__ __noinline__ void sweep_pairs_mixed() {
     reduce_to_P<KH, TPL>(ar, ai, sm, c0);
 }
 
+// Shared memory a variant's kernels with a sweep set aside for the tables, over the draw's weights.
+template <int TPL, int KPM, int PREC>
+constexpr size_t pair_table_bytes() {
+    if (PREC == PREC_COMP || !has_pairs<TPL, KPM>()) return 0;
+    return PREC == PREC_MIXED ? sizeof(PairTables32<NARROW>) : sizeof(PairTables<NARROW>);
+}
+
 }  // namespace pe

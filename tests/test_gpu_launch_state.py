@@ -81,3 +81,12 @@ def test_two_threads_with_different_mode_counts():
     for t in threads:
         t.join()
     assert not errors
+
+
+def test_only_variants_with_the_pair_sweep_set_its_tables_aside():
+    """FP64 CTAs of one warp, bound by shared memory: two-thread lanes at 16 columns have no pair sweep, one-thread lanes
+    do, and their 16.5 KB of tables cost them a CTA per SM (38 KB of layout: five without, four with)."""
+    from photonic_engines_b200 import _native as N
+    L = N.load()
+    with_tables, without = (L.pe_split_slots(N.PRECISIONS["f64"], 16, 32, tpl) for tpl in (1, 2))
+    assert 0 < with_tables < without
