@@ -24,6 +24,7 @@ static __device__ __forceinline__ void load_rows(SM& sm, const double2* __restri
 // exchange carries half of the values still held.
 template <int KH, class WS>
 __device__ __forceinline__ void cofactors_direct_kh(WS& sm, int K) {
+    static_assert(KH <= 5, "the reduction over the lanes knows halves of one or two columns and odd KH");
     const int lid = threadIdx.x & 31, h = lid & 1, c0 = h * KH, K1 = K - 1;
     const int N = 1 << (K1 - 1);
     double ar[KH], ai[KH];
@@ -108,15 +109,15 @@ __device__ __forceinline__ void cofactors_direct_kh(WS& sm, int K) {
 }
 
 template <int KMAX, class WS>
-__device__ __forceinline__ void cofactors_direct(WS& sm, int K) {
+__device__ __forceinline__ void cofactors_direct(WS& sm, int K) {             // K <= KMAX
     if (K <= 4) { cofactors_direct_kh<2>(sm, K); return; }
     if (K <= 6) { cofactors_direct_kh<3>(sm, K); return; }
     if constexpr (KMAX <= 8) {
         cofactors_direct_kh<4>(sm, K);
     } else {
+        static_assert(KMAX <= 10, "five columns per thread at most");
         if (K <= 8) cofactors_direct_kh<4>(sm, K);
-        else if (K <= 10) cofactors_direct_kh<5>(sm, K);
-        else cofactors_direct_kh<6>(sm, K);
+        else cofactors_direct_kh<5>(sm, K);
     }
 }
 

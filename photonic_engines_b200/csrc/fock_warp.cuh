@@ -500,7 +500,7 @@ __device__ void chain_warp(const ChainParams& p, WS& sm, int64_t s) {
             if (lane == 0) sm.P[0] = make_double2(1.0, 0.0);
             __syncwarp();
         } else if (direct) {
-            cofactors_direct<KPW>(sm, k);
+            cofactors_direct<WDIRECT<KPW, MIXED>>(sm, k);
         } else if constexpr (KPW > WDIRECT<KPW, MIXED>) {
             build_groups_warp(sm, K1);
             __syncwarp();
