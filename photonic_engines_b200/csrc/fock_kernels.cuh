@@ -221,6 +221,10 @@ template <class SM>
 __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid_max, int pair_lanes = 0,
                           int pair_lin = 0, int pair_min = 2) {
     auto& pl = sm.plan;
+    // scratch: active digits by ascending radix, over the inner weights (the last step's, no longer read)
+    int* const sortR = reinterpret_cast<int*>(sm.tab_w);
+    int* const sortG = sortR + SM::NKMAX;
+    static_assert(sizeof(sm.tab_w) >= 2 * SM::NKMAX * sizeof(int), "the planner's scratch");
     constexpr int GL = (SM::NKMAX + 31) / 32;          // groups (and ranks) per lane: index lane + 32 q, q < GL
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -277,8 +281,8 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
             const unsigned eq = __ballot_sync(full, take);
             if (take) {
                 const int r = na + __popc(eq & below);
-                pl.sortR[r] = (unsigned char)R[q];
-                pl.sortG[r] = (unsigned char)(lane + 32 * q);
+                sortR[r] = R[q];
+                sortG[r] = lane + 32 * q;
             }
             na += __popc(eq);
             rem[q] &= ~eq;
@@ -291,8 +295,8 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
 #pragma unroll
     for (int q = 0; q < GL; ++q) {
         const int p = lane + 32 * q;
-        rv[q] = p < na ? (TC)pl.sortR[p] : TC(1);
-        gp[q] = p < na ? pl.sortG[p] : 0;
+        rv[q] = p < na ? (TC)sortR[p] : TC(1);
+        gp[q] = p < na ? sortG[p] : 0;
         mp[q] = p < na ? sm.gmul[gp[q]] : 1;
         pre[q] = rv[q];
     }
@@ -360,8 +364,8 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
             pl.R[kd] = (int)rv[q];
             pl.M[kd] = mp[q];
             pl.drow[kd] = sm.grow[gp[q]];
-            if (p >= nhi && p < nhi + nin) pl.Pin[kd] = (unsigned short)pin[q];
-            if (p >= nhi + nin && p < nhi + nin + nmid) pl.Pmid[kd - nin] = (unsigned short)pmid[q];
+            if (p >= nhi && p < nhi + nin) pl.Pin[kd] = pin[q];
+            if (p >= nhi + nin && p < nhi + nin + nmid) pl.Pmid[kd - nin] = pmid[q];
         }
         const int g = lane + 32 * q;                   // fixed digits: after the active ones, in group order
         const bool fixed = g < D && !active[q] && g != gu && g != gv;
@@ -397,7 +401,7 @@ __device__ void plan_step(SM& sm, int K1, int K, int lanes, int lin_max, int mid
 // ones: every digit has radix 2 and multiplicity 1, so the digits are the bits of the Gray code of t and the
 // weight its parity.  vend (optional): the digit values at t.
 template <class PL>
-static __device__ __forceinline__ unsigned char gray_entry(const PL& pl, int d0, int nd, const unsigned short* Pp, int t,
+static __device__ __forceinline__ unsigned char gray_entry(const PL& pl, int d0, int nd, const int* Pp, int t,
                                                           double* w_out, unsigned char* vend, bool ones) {
     if (ones) {
         const int g = t ^ (t >> 1);

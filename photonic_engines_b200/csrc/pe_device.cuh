@@ -77,14 +77,12 @@ struct PlanT {
     int R[NK];        // radix per kernel digit
     int M[NK];        // multiplicity per kernel digit
     int drow[NK];     // output mode per kernel digit
-    unsigned short Pin[NK];   // prefix products of the inner radices (at most LIN_MAX)
-    unsigned short Pmid[NK];  // prefix products of the middle radices (at most MID_MAX)
+    int Pin[NK];      // prefix products of the inner radices
+    int Pmid[NK];     // prefix products of the middle radices
     unsigned char vend[NK];   // inner digit values after a forward inner block
     int ones_in, ones_mid;   // the schedules' digits all have radix 2 and multiplicity 1
     int pairs;        // two digits are taken out of the walk as u, v of the pair sweep (fock_pairs.cuh)
     int pu, pv;       // their kernel digits
-    unsigned char sortR[NK];  // scratch of the planner: active digits by ascending radix (radices up to NK), their groups
-    unsigned char sortG[NK];
 };
 
 // Precision forms (the values of PE_PRECISION_* in pe_b200.h)
@@ -146,6 +144,5 @@ __host__ __device__ constexpr size_t smem_fixed_bytes_for(int kpm, int prec = PR
 static_assert(smem_fixed_bytes<NARROW>() <= 46800 && smem_fixed_bytes<NARROW, PREC_MIXED>() <= 46800, "modes, FP64 and mixed");
 static_assert(smem_fixed_bytes<NARROW, PREC_COMP>() <= 54992, "modes, compensated");
 static_assert(smem_fixed_bytes<MAXN>() <= 93824, "modes, 33 to 64 photons");
-static_assert(LIN_MAX < 65536 && MID_MAX < 65536 && MAXN < 256, "the plan's short fields");
 
 }  // namespace pe
