@@ -16,11 +16,13 @@ import torch
 from .. import _native as N
 
 
-def pack_instances(U: torch.Tensor, in_modes) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
+def pack_instances(U: torch.Tensor, in_modes, copy: bool = True) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """U [B, m, m] (or [m, m]) and the n input modes -> (acol, inst_off, inst_m, inst_n).
 
     Instance b holds the n input columns U[b][:, in_modes] column-major: acol[b, j, rho] = U[b, rho, in_modes[j]],
-    complex128, so that one input column is m contiguous complex values.
+    complex128, so that one input column is m contiguous complex values.  copy=False: acol may be U's own memory where
+    that already has this layout (column-major circuits, as torch.linalg.qr returns them), for callers that are done
+    with it before they hand U back.
     """
     if U.dim() == 2:
         U = U[None]
@@ -32,10 +34,12 @@ def pack_instances(U: torch.Tensor, in_modes) -> tuple[torch.Tensor, torch.Tenso
         cols = U[:, :, modes[0]:modes[0] + n]                # a run of modes: no index tensor to copy over
     else:
         cols = U[:, :, torch.tensor(modes, dtype=torch.int64, device=dev)]
-    # a copy of its own whatever U is: a run's slice may already lie in this layout (U.mH, U.mT), and then
-    # contiguous() would hand back U's memory, with its conjugation flag
-    acol = torch.empty(B, n, m, dtype=torch.complex128, device=dev)
-    acol.copy_(cols.transpose(1, 2))
+    cols = cols.transpose(1, 2)                              # [B, n, m]
+    if not copy and cols.dtype == torch.complex128 and cols.is_contiguous() and not cols.is_conj() \
+            and not cols.is_neg() and cols.data_ptr() % 16 == 0:                # the kernels load 16 bytes at a time
+        acol = cols
+    else:
+        acol = cols.to(torch.complex128, memory_format=torch.contiguous_format, copy=True)     # resolves the flags
     inst_off = torch.arange(0, B * n * m, n * m, dtype=torch.int64, device=dev) if n * m > 0 else \
         torch.zeros(B, dtype=torch.int64, device=dev)
     inst_m = torch.full((B,), m, dtype=torch.int32, device=dev)
@@ -170,7 +174,10 @@ def split_shape(heavy_streams: int, n: int, device, block_threads: int = 0, tpl:
     its steps (up to 32 photons, FP64 and mixed forms): a step's work shrank but not what a CTA spends on its plan,
     so a stream gets no more CTAs than fill PAIR_FILL waves (PAIR_FILL_LONG at 24-26 photons), nor so many that a
     lane of the last step walks fewer than PAIR_BLOCKS_PER_LANE blocks, unless SMs would stay idle; k_split is the
-    first step with eight blocks per lane (one for fewer than 16 streams)."""
+    first step with eight blocks per lane (one for fewer than 16 streams).  A caller's lane width without the pair
+    sweep (four threads, or two up to 20 photons) takes the same shape: its steps run term by term, but split_plan's
+    CTAs cost it their planning too (FP64 ms, split_plan -> here: n = 20, m = 400, 32 streams, two threads 0.98 ->
+    0.73, four 0.97 -> 0.87; four threads, n = 24, m = 48, 512 streams 26.2 -> 24.6, 64 streams 8.0 -> 6.2)."""
     plan = split_plan(heavy_streams, n, device, block_threads, tpl, precision)
     if plan is None or n > N.PE_MIXED_MAX_PHOTONS or precision == "compensated" or n < 17:
         return plan

@@ -89,7 +89,7 @@ def sample_chains(U, in_modes, sigma, *, uniforms=None, seeds=None, seed_row=Non
     S, n = sigma.shape
     if dp is None:
         dp = torch.zeros(S, dtype=torch.int64, device=dev)
-    acol, inst_off, inst_m, inst_n = pack_instances(U, in_modes)
+    acol, inst_off, inst_m, inst_n = pack_instances(U, in_modes, copy=False)
     if split is None:
         split = split_shape(S, n, dev, block_threads, tpl or default_tpl(n, precision), precision)
     rows, occ, marg = chain(acol, inst_off, inst_m, inst_n, dp, sigma, m_max=U.shape[1], uniforms=uniforms, seeds=seeds,
@@ -191,7 +191,7 @@ def fock_sample(U, in_modes, shots, generator=None, algo="auto", multi_min_k1=10
         return _adaptive(U, in_modes, S, dp_all, generator, max_streams, prefix, avoid, keep_ids, stats,
                          precision, uniforms, block_threads, tpl)
     plan = plan_chains(U, in_modes, S, dp_all, generator, loss, d, max_streams, _index=False)
-    acol, inst_off, inst_m, inst_n = pack_instances(U, in_modes)
+    acol, inst_off, inst_m, inst_n = pack_instances(U, in_modes, copy=False)
     t0 = None
     if stats is not None:
         torch.cuda.synchronize(dev)
@@ -260,7 +260,7 @@ def _adaptive(U, in_modes, S, dp_all, generator, max_streams, prefix, avoid, kee
     if avoid is not None:
         mask = torch.zeros(m, dtype=torch.uint8, device=dev)
         mask[avoid] = 1
-    acol, inst_off, inst_m, inst_n = pack_instances(U, in_modes)
+    acol, inst_off, inst_m, inst_n = pack_instances(U, in_modes, copy=False)
     u = None if uniforms is None else torch.as_tensor(uniforms, dtype=torch.float64, device=dev)
     t0 = None
     if stats is not None:

@@ -29,5 +29,22 @@ def test_packed_columns_are_a_resolved_copy(view, dtype, batch, modes):
     assert torch.equal(acol, want)
     torch.view_as_real(acol)                                     # what the launches pass on
     assert acol.numel() == 0 or acol.untyped_storage().data_ptr() != U.untyped_storage().data_ptr()
+    shared = pack_instances(U, modes, copy=False)[0]
+    assert shared.dtype == torch.complex128 and shared.is_contiguous() and not shared.is_conj() and not shared.is_neg()
+    assert torch.equal(shared, want)
     assert off.tolist() == [b * len(modes) * 6 for b in range(max(batch, 1))]
     assert mm.tolist() == [6] * max(batch, 1) and nn.tolist() == [len(modes)] * max(batch, 1)
+
+
+def test_shared_columns_are_the_circuits_memory_only_where_the_kernels_can_read_it():
+    """The kernels load 16 bytes at a time: a column-major circuit at an odd multiple of 8 bytes is copied."""
+    n, m = 3, 6
+    buf = torch.randn(2 * m * m + 4, dtype=torch.float64)
+    first = (buf.data_ptr() // 8) % 2                            # 16-byte aligned start, in doubles
+    for shift in (0, 1):
+        raw = buf.numpy()[first + shift:][:2 * m * m]
+        U = torch.from_numpy(raw.view("complex128").reshape(m, m)).mT
+        assert U.data_ptr() % 16 == 8 * shift
+        acol = pack_instances(U, range(n), copy=False)[0]
+        assert (acol.data_ptr() == U.data_ptr()) == (shift == 0) and acol.data_ptr() % 16 == 0
+        assert torch.equal(acol[0], U[:, :n].mT)
