@@ -418,7 +418,9 @@ def run_b200(args):
                     "algorithmic_bytes_per_launch": statistics.mean(w["bytes"] for w in r["work"]),
                     "peak_source": "measured live by pe_pipe_probe (FMA chains) on this GPU; nominal = lanes x 2 "
                                    "x 148 SMs x SM clock",
-                    "flops_per_launch": flops_launch, "launch_ms": dur * 1e3}
+                    "flops_per_launch": flops_launch, "launch_ms": dur * 1e3,
+                    "flops_rule": "22 per column and term of the collapsed sum, term by term; the FP64 and mixed pair "
+                                  "sweep executes about 15, so frac overstates how busy the pipe is"}
 
         forms = {f: {"value": value[f], "ms_per_step": res[f]["elapsed"] / args.steps * 1e3,
                      "roofline": roof(res[f], f), "max_marginal_rel_err": err[f], "meets_bound": meets[f],
