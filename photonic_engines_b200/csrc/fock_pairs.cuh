@@ -14,7 +14,7 @@
 // table G holds their steps); S multiplies the column sums once per block, X_u and X_v only once per sweep.
 // Per pair and term that is 5 FP64 instructions for the products, 12 for the all-but-one products over the
 // pairs (prefix, suffix, accumulation) and 4 for the rest: 21, against 28 for two columns taken one by one.
-// Bound by the FP64 pipe (70-75 % busy inside the sweep).  Lanes of two threads with ten columns each at 20 columns
+// Bound by the FP64 pipe (68-69 % busy inside the sweep).  Lanes of two threads with ten columns each at 20 columns
 // (eleven doubles of state per column pair and thread: 255 registers with a few spills to L1), of four threads with
 // six to eight beyond.  Measured against the term-by-term sweep: n = 20, m = 400, 2 000 streams 18.3 -> 14.2 ms;
 // n = 24, m = 576, 600 streams 128 -> 97 ms; cofactors at 28 columns (148 blocks) 329 -> 274 ms, at 32 columns
