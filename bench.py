@@ -312,6 +312,10 @@ def run_b200(args):
         for _ in range(warmup):
             step(precision)
         torch.cuda.synchronize(dev)
+        # the rows kept below come out of the allocator's cache: a cudaMalloc inside the timed region can wait 50 to
+        # 100 ms for the clock sampler's nvidia-smi to start, with the GPU idle
+        held = [torch.empty(SHOTS, N_PHOT, dtype=torch.int64, device=dev) for _ in range(steps + 1)]
+        del held
         kern_ms, work, all_rows = [], [], []
         barrier()
         torch.cuda.synchronize(dev)
